@@ -48,7 +48,13 @@ struct ProbDev {
   // TMA tensor maps over them (TcMaps, in the call header)
   const void* xh;
   const void* yh;
-  const void* maps;
+  union {
+    const void* maps;
+    // FP32 row-owner engine, grid team: exchange words {FP32 potential, sweep
+    // number} of x [n] and of both g buffers [2][m], or null (potentials
+    // exchanged through f and gbuf behind a barrier)
+    unsigned long long* words;
+  };
   // tensor-core path: column-shift rows [pad][8] bf16 of x and [2][pad][8]
   // of y (one per g buffer), written by every potential update
   void* extx;
@@ -118,8 +124,7 @@ struct Sched {
 };
 
 struct Globals {
-  unsigned int bar_count;
-  unsigned int bar_gen;
+  unsigned long long bar_count;  // grid_barrier arrivals so far
   unsigned int unit_ctr[3];
   int pad_;
 };
@@ -181,6 +186,11 @@ __device__ __forceinline__ void unpack2(f32x2 r, float& a, float& b) {
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   f32x2 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
@@ -257,6 +267,8 @@ __device__ __forceinline__ f32x2 exp2_poly2_d4(f32x2 xp) {
 #ifndef OTTB_POLY_OF_8
 #define OTTB_POLY_OF_8 2
 #endif
+// The row-owner engine at d <= 4: of every 16 pairs of exponentials.
+__host__ __device__ constexpr int rows_poly_pairs(int D) { return D <= 2 ? 2 : D == 3 ? 1 : 0; }
 #ifndef OTTB_POLY_OF_8_TC
 #define OTTB_POLY_OF_8_TC 2
 #endif
@@ -324,39 +336,57 @@ __device__ __forceinline__ void lse_merge(float& m, float& l, float m2, float l2
   m = mx;
 }
 
-// Grid-wide barrier for a cooperative (co-resident) grid. The wait is
-// bounded: after deadline_ns of waiting the CTA records OTTB_ERR_TIMEOUT in
-// *status and returns false. expected = gridDim.x + phantom arrivals.
+// Grid-wide barrier for a cooperative (co-resident) grid: one counter that
+// only grows, one arrival (a release) per CTA and phase, and a spin on its
+// value (an acquire). GridBarrier is the CTA's phase, kept by thread 0. The wait is bounded:
+// after timeout_ns the CTA records OTTB_ERR_TIMEOUT in *status, poisons the
+// counter, so that every other CTA leaves its wait too, and returns false.
+// expected = gridDim.x + phantom arrivals. A counter that the last arriver
+// resets and a generation that the others poll with a sleep took ~4900
+// cycles for the last arriver alone (four dependent atomics and a status
+// read); this takes one atomic and one poll.
+struct GridBarrier {
+  unsigned long long phase;
+};
+
+constexpr unsigned long long kBarrierPoison = 1ull << 62;
+
+// Ends every CTA's wait at a barrier with false (after a timeout elsewhere).
+__device__ __forceinline__ void grid_abort(Globals* gl, int* status) {
+  atomicExch(status, (int)OTTB_ERR_TIMEOUT);
+  __threadfence();
+  atomicOr(&gl->bar_count, kBarrierPoison);
+}
+
 __device__ __forceinline__ bool grid_barrier(Globals* gl, unsigned expected,
-                                             uint64_t timeout_ns, int* status) {
-  __syncthreads();
+                                             uint64_t timeout_ns, int* status,
+                                             GridBarrier& bar) {
   __shared__ int s_ok;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    volatile unsigned* vgen = &gl->bar_gen;
-    unsigned gen = *vgen;
-    __threadfence();
-    unsigned arrived = atomicAdd(&gl->bar_count, 1u);
-    int ok = 1;
-    if (arrived == expected - 1) {
-      atomicExch(&gl->bar_count, 0u);
-      __threadfence();
-      atomicAdd(&gl->bar_gen, 1u);
-    } else {
-      uint64_t t0 = global_timer_ns();
-      unsigned ns = 32;
-      while (*vgen == gen) {
-        __nanosleep(ns);
-        if (ns < 256) ns <<= 1;
-        if (global_timer_ns() - t0 > timeout_ns) {
-          ok = 0;
-          atomicExch(status, (int)OTTB_ERR_TIMEOUT);
+    const unsigned long long target = ++bar.phase * expected;
+    // release and acquire at gpu scope are cumulative over the CTA's
+    // __syncthreads: no separate fences
+    unsigned long long* ctr = &gl->bar_count;
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(ctr) : "memory");
+    auto poll = [&]() {
+      unsigned long long v;
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ctr) : "memory");
+      return v;
+    };
+    unsigned long long v = poll();
+    if (v < target) {
+      const uint64_t t0 = global_timer_ns();
+      int spin = 0;
+      while ((v = poll()) < target) {
+        if ((++spin & 63) == 0 && global_timer_ns() - t0 > timeout_ns) {
+          grid_abort(gl, status);
+          v = kBarrierPoison;
           break;
         }
       }
     }
-    __threadfence();
-    if (ok && *((volatile int*)status) == OTTB_ERR_TIMEOUT) ok = 0;
-    s_ok = ok;
+    s_ok = v < kBarrierPoison;
   }
   __syncthreads();
   return s_ok != 0;

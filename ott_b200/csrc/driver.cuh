@@ -49,7 +49,7 @@ struct SweepParams {
 
 __device__ __forceinline__ float eps_mult(const ottb_solver_cfg& c, int it) {
   // epsilon_scheduler.py:47-60: max(init * decay^it, 1)
-  float mlt = c.eps_init * powf(c.eps_decay, (float)it);
+  float mlt = c.eps_decay == 1.0f ? c.eps_init : c.eps_init * powf(c.eps_decay, (float)it);
   return fmaxf(mlt, 1.0f);
 }
 

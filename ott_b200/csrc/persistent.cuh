@@ -275,6 +275,7 @@ __device__ void persistent_main(const KernelArgs& A, SweepFn&& sweep) {
   const bool force_scan = c.min_iterations == c.max_iterations;
   const int scan_end = force_scan ? (c.max_iterations / inner) * inner : c.max_iterations;
   int* status = &A.sched->status;
+  GridBarrier bar{0};
   unsigned sweep_idx = 0;
   int it = 0;
   int commits = 0;  // committed g-sweeps; identical in every CTA
@@ -305,14 +306,13 @@ __device__ void persistent_main(const KernelArgs& A, SweepFn&& sweep) {
   do {                                                                           \
     begin_sweep(sp);                                                             \
     if (!sweep((sp), sweep_idx++)) {                                             \
-      if (threadIdx.x == 0) atomicExch(status, (int)OTTB_ERR_TIMEOUT);           \
-      grid_barrier(A.gl, A.expected_arrivals, A.timeout_ns, status);             \
+      if (threadIdx.x == 0) grid_abort(A.gl, status);                            \
       return;                                                                    \
     }                                                                            \
   } while (0)
 #define OTTB_BARRIER()                                                          \
   do {                                                                          \
-    if (!grid_barrier(A.gl, A.expected_arrivals, A.timeout_ns, status)) return; \
+    if (!grid_barrier(A.gl, A.expected_arrivals, A.timeout_ns, status, bar)) return; \
   } while (0)
 
   if (c.init_f_from_g && scan_end > 0) {
