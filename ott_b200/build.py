@@ -42,7 +42,7 @@ def up_to_date(out, deps) -> bool:
 def _nvcc_shared(srcs, out, verbose):
   os.makedirs(OUT_DIR, exist_ok=True)
   srcs = [srcs] if isinstance(srcs, str) else list(srcs)
-  cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
+  cmd = [nvcc(), *ARCH, "--threads", "0", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
          "-shared", "-o", out + ".tmp", *srcs]
   if verbose:
     cmd.insert(1, "-Xptxas=-v")
@@ -60,7 +60,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
   if force or not up_to_date(OUT, deps):
     _nvcc_shared([os.path.join(CSRC, "capi.cu"), os.path.join(CSRC, "noalloc.cu"),
                   os.path.join(CSRC, "mlp.cu"), os.path.join(CSRC, "transport.cu"),
-                  os.path.join(CSRC, "transport_tc.cu"),
+                  os.path.join(CSRC, "transport_tc.cu"), os.path.join(CSRC, "rows.cu"),
                   os.path.join(CSRC, "krylov.cu")], OUT,
                  verbose)
   peaks = os.path.join(CSRC, "peaks", "peaks.cu")

@@ -114,6 +114,7 @@ struct InitArgs {
   const float* const* init;  // [2 * P]: f_init_p, g_init_p (may be null)
   ProbDev* probs;
   int mask;                  // mask caller init with -inf at zero weights
+  int rows;                  // row-owner engine: clear its exchange words and keys
 };
 
 __global__ void init_potentials_kernel(InitArgs args) {
@@ -125,6 +126,12 @@ __global__ void init_potentials_kernel(InitArgs args) {
   // f over n_pad, then g over both g buffers' m_pad rows (padding rows get
   // the -inf column shift of the tensor-core path)
   const int64_t tot = P.n_pad + 2 * P.m_pad;
+  if (args.rows && P.dkey && blockIdx.x == 0 && threadIdx.x < 8)
+    P.dkey[threadIdx.x] = (threadIdx.x & 1) ? kDkeyEmptyMin : kDkeyEmptyMax;
+  if (args.rows && P.words)
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.n + 2 * P.m;
+         i += (int64_t)gridDim.x * blockDim.x)
+      P.words[i] = 0ull;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < tot;
        i += (int64_t)gridDim.x * blockDim.x) {
     if (i < P.n_pad) {

@@ -22,6 +22,8 @@
 #include "aux_kernels.cuh"
 #include "kernel_simt.cuh"
 #include "kernel_tc.cuh"
+#include "launch.cuh"
+#include "rows.h"
 #include "tmap.cuh"
 
 using namespace ottb;
@@ -62,7 +64,7 @@ int simt_dp(int d) {
   return dp;
 }
 
-// Kernel table for the CUDA-core engine.
+// Kernel table for the tiled CUDA-core engine (d > 4; see rows_wanted).
 template <int DP>
 struct SimtKernel {
   static void* fn() { return (void*)&sinkhorn_simt_kernel<DP>; }
@@ -78,8 +80,6 @@ struct KernelChoice {
 KernelChoice pick_simt(int dp) {
   KernelChoice k;
   switch (dp) {
-    case 2: k.fn = SimtKernel<2>::fn(); k.smem = SimtKernel<2>::smem(); break;
-    case 4: k.fn = SimtKernel<4>::fn(); k.smem = SimtKernel<4>::smem(); break;
     case 8: k.fn = SimtKernel<8>::fn(); k.smem = SimtKernel<8>::smem(); break;
     case 16: k.fn = SimtKernel<16>::fn(); k.smem = SimtKernel<16>::smem(); break;
     case 32: k.fn = SimtKernel<32>::fn(); k.smem = SimtKernel<32>::smem(); break;
@@ -228,6 +228,8 @@ struct ProbPlan {
   int rb_f, rb_g, split_f, split_g, smax_f, smax_g;
   size_t off_xt, off_yt, off_nx, off_ny, off_galt, off_pm, off_pl, off_arr, off_err,
       off_msum, off_extx, off_exty, off_cen, off_lprev;
+  // row-owner engine, grid team: the exchanged values and the keys fit
+  bool words = false, keys = false;
 };
 
 // BF16 split-3 on tcgen05 when asked for, and by default where the inner
@@ -237,8 +239,23 @@ bool wants_tc(const ottb_solver_cfg* cfg, int d) {
   return cfg->precision == OTTB_PRECISION_AUTO && d >= 32;
 }
 
+// How the row-owner engine runs an FP32 call (engine_rows.cuh, rows_wanted). The problems of `cluster` are drawn by thread-block
+// clusters of `csize` CTAs, those of `grid` are solved one after another by
+// the whole grid; both are table positions in decreasing work.
+struct RowsPlan {
+  bool on = false;
+  RowsKernel kern;
+  std::vector<int> cluster, grid;
+  int csize = 1, cthreads = 0, nclusters = 0;
+  size_t csmem = 0;
+  int gsize = 0;
+  bool resident = false, seqwords = false;
+  size_t gsmem = 0;
+};
+
 struct Plan {
   int num = 0;
+  RowsPlan rows;
   int dp = 0;        // FP32 engine: padded dimension; tensor cores: DK
   bool tc = false;
   int grid = 0;
@@ -308,6 +325,159 @@ int validate_cfg(const ottb_solver_cfg* cfg) {
   return OTTB_OK;
 }
 
+// Whether an FP32 call goes to the row-owner engine rather than the tiled
+// one: always at d <= 4, where the tiled engine's loop is bound by its issue
+// slots (n = m = 16000, d = 2: 6.2 against 7.8 ms; n = 7013, m = 5001, d =
+// 3: 5.2 against 11); above, while the points stay in shared memory or, for
+// one problem at d <= 10, also streamed (n = m = 16000, d = 10: 13.3 against
+// 16.8 ms; d = 16: 20.5 against 16.8). A batch goes there when each of its
+// problems fits a cluster of 8 (96 problems up to 4096 points, d = 8, of
+// which a part had to go through the grid one by one: 12.8 against 7.6).
+bool rows_wanted(const ottb_problem* probs, int num, int d) {
+  const int D = rows_kernel(d).D;
+  if (D == 0) return false;
+  if (D <= 4 || (num == 1 && D <= 10)) return true;
+  constexpr size_t kFits = 224 * 1024;
+  if (num == 1)
+    return rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true) <= kFits;
+  for (int i = 0; i < num; ++i)
+    if (rows_smem(probs[i].n, probs[i].m, D, 8, kRowsWarps, true, false) > kFits) return false;
+  return true;
+}
+
+// Dynamic shared memory a row-owner CTA may ask for (227 KB less its static
+// part).
+const size_t kRowsSmemMax = 227 * 1024 - rows_static_smem() - 64;
+
+// Clusters of `size` CTAs that the device holds at once. Cached: the query
+// stays out of later calls, which may be under stream capture.
+int rows_max_clusters(const void* fn, int size, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int, int, size_t>, int> cache;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(dev, fn, size, threads, smem);
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return 0;
+  cudaLaunchConfig_t lc;
+  std::memset(&lc, 0, sizeof(lc));
+  lc.gridDim = dim3(size);
+  lc.blockDim = dim3(threads);
+  lc.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, fn, &lc) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  if (cache.size() > 4096) cache.clear();
+  cache[key] = n;
+  return n;
+}
+
+// Team sizes of the row-owner engine, from a model of one sweep in SM
+// cycles: entries x cycles per entry / CTAs, plus what a sweep costs beyond
+// its entries (column shifts, lane and warp merges, the update in FP64, the
+// team's barrier).
+int plan_rows(Plan& plan, int d, const DeviceInfo& di) {
+  RowsPlan& R = plan.rows;
+  R.kern = rows_kernel(d);
+  const int D = R.kern.D;
+  const double per_entry = D <= 4 ? 0.105 : (D + 8) / 75.0;
+  const double over_one = 4500, over_cluster = 5500, over_grid = 11000, over_warp = 100;
+  const int num = plan.num;
+  if (!ensure_dynamic_smem(R.kern.grid, kRowsSmemMax) ||
+      !ensure_dynamic_smem(R.kern.cluster, kRowsSmemMax))
+    return OTTB_ERR_CUDA;
+  // grid: as many CTAs as there are quads of rows, and as the per-CTA sums
+  // have room for in the workspace
+  auto grid_size = [&](const ProbPlan& pp) {
+    int64_t g = std::min<int64_t>(std::min(di.sms, kRowsMaxCtas), (std::max(pp.n, pp.m) + 3) / 4);
+    const int64_t slots = (int64_t)std::min<size_t>(pp.off_arr - pp.off_pm, kRowsKeyBytes) / 16;
+    return (int)std::max<int64_t>(1, std::min(g, std::max<int64_t>(pp.rb_g, slots)));
+  };
+  auto entries = [&](const ProbPlan& pp) { return (double)pp.n * (double)pp.m * per_entry; };
+  // cost[k]: the k largest problems by the whole grid, the rest by clusters
+  std::vector<double> grid_t(num + 1, 0.0);
+  for (int t = 0; t < num; ++t)
+    grid_t[t + 1] = grid_t[t] + entries(plan.probs[t]) / grid_size(plan.probs[t]) + over_grid;
+  double best = grid_t[num];
+  int best_k = num;
+  for (int C = 1; C <= kRowsMaxCluster; C *= 2) {
+    for (int threads = kRowsThreads; threads >= 128; threads /= 2) {
+      const int warps = threads / 32;
+      double sum = 0.0, longest = 0.0;
+      size_t smem = 0;
+      for (int k = num - 1; k >= 0; --k) {
+        const ProbPlan& pp = plan.probs[k];
+        smem = std::max(smem, rows_smem(pp.n, pp.m, D, C, warps, true, false));
+        if (smem > kRowsSmemMax) break;
+        // CTAs that share an SM share its pipes; one alone needs about ten
+        // warps to fill them
+        const int per_sm = std::min<int>(kRowsThreads / threads,
+                                         (int)(kRowsSmemMax / (smem + rows_static_smem() + 1024)));
+        // large clusters leave SMs of a GPC over (7 of 9 clusters of 16 fit)
+        const double slots = (double)di.sms * std::max(per_sm, 1) / C *
+                             (C >= 8 ? 0.78 : C >= 4 ? 0.88 : 1.0);
+        const double alone = std::min(1.0, warps / 10.0);
+        const double share = std::max(1.0, std::min((double)per_sm, (num - k) * C / (double)di.sms));
+        const double t = entries(pp) / C / std::min(alone, 1.0 / share) +
+                         (C > 1 ? over_cluster : over_one) + over_warp * warps;
+        sum += t;
+        longest = std::max(longest, t);
+        // problems stop at different iterations: a batch ends with its
+        // longest-running ones
+        const double est = num - k == 1 ? t : std::max(longest, sum / slots + longest);
+        if (grid_t[k] + est < best) {
+          best = grid_t[k] + est;
+          best_k = k;
+          R.csize = C;
+          R.cthreads = threads;
+          R.csmem = smem;
+        }
+      }
+    }
+  }
+  R.grid.clear();
+  R.cluster.clear();
+  for (int t = 0; t < num; ++t) (t < best_k ? R.grid : R.cluster).push_back(t);
+  if (!R.cluster.empty()) {
+    R.nclusters = rows_max_clusters(R.kern.cluster, R.csize, R.cthreads, R.csmem);
+    if (R.nclusters < 1) return OTTB_ERR_CUDA;
+    R.nclusters = std::min<int>(R.nclusters, (int)R.cluster.size());
+  }
+  if (!R.grid.empty()) {
+    R.gsize = di.sms;
+    for (int t : R.grid) R.gsize = std::min(R.gsize, grid_size(plan.probs[t]));
+    size_t res = 0, str = 0;
+    for (int t : R.grid) {
+      const ProbPlan& pp = plan.probs[t];
+      res = std::max(res, rows_smem(pp.n, pp.m, D, R.gsize, kRowsWarps, false, true));
+      str = std::max(str, rows_smem(pp.n, pp.m, D, R.gsize, kRowsWarps, false, false));
+    }
+    R.resident = res <= kRowsSmemMax;
+    R.seqwords = R.resident;
+    R.gsmem = R.resident ? res : str;
+    if (R.gsmem > kRowsSmemMax) return OTTB_ERR_UNSUPPORTED;
+    for (int t : R.grid) {
+      ProbPlan& pp = plan.probs[t];
+      pp.keys = kRowsSumBytes <= pp.off_arr - pp.off_pm;
+      pp.words = rows_words_bytes(pp.n, pp.m) <= pp.off_arr - pp.off_pm;
+      R.seqwords = R.seqwords && pp.words && pp.n + pp.m <= kRowsWordsMax;
+    }
+  }
+  R.on = true;
+  return OTTB_OK;
+}
+
 // The work plan of a call. sched_override (or else the autotune cache, or
 // else the defaults) sets the schedule knobs; the workspace layout does not
 // depend on them.
@@ -319,19 +489,28 @@ int make_plan(const ottb_problem* probs, int num, int d, const ottb_solver_cfg* 
   if (d > 128) return OTTB_ERR_UNSUPPORTED;
   plan.num = num;
   plan.tc = wants_tc(cfg, d);
+  bool rows = false;
+  for (int i = 0; i < num; ++i) {
+    if (probs[i].n < 1 || probs[i].m < 1) return OTTB_ERR_INVALID;
+    if (probs[i].n > (int64_t)1 << 31 || probs[i].m > (int64_t)1 << 31) return OTTB_ERR_UNSUPPORTED;
+  }
   if (plan.tc) {
     plan.dp = d <= 64 ? 64 : 128;
     plan.kern = pick_tc(plan.dp, 256);
   } else {
     plan.dp = simt_dp(d);
-    plan.kern = pick_simt(plan.dp);
+    rows = rows_wanted(probs, num, d);
+    if (rows)
+      plan.kern.fn = const_cast<void*>(rows_kernel(d).grid);
+    else
+      plan.kern = pick_simt(plan.dp);
   }
   if (!plan.kern.fn) return OTTB_ERR_UNSUPPORTED;
   if (need_grid) {
     DeviceInfo di = device_info();
     if (di.sms <= 0) return OTTB_ERR_NO_DEVICE;
     if (di.major < 10) return OTTB_ERR_NO_DEVICE;
-    plan.grid = persistent_grid(plan.kern, di.sms);
+    plan.grid = rows ? di.sms : persistent_grid(plan.kern, di.sms);
     if (plan.grid <= 0) return OTTB_ERR_CUDA;
   } else {
     plan.grid = 148;
@@ -339,11 +518,7 @@ int make_plan(const ottb_problem* probs, int num, int d, const ottb_solver_cfg* 
   // Problems ordered by decreasing work so the atomic queue deals the
   // largest units first.
   plan.order.resize(num);
-  for (int i = 0; i < num; ++i) {
-    if (probs[i].n < 1 || probs[i].m < 1) return OTTB_ERR_INVALID;
-    if (probs[i].n > (int64_t)1 << 31 || probs[i].m > (int64_t)1 << 31) return OTTB_ERR_UNSUPPORTED;
-    plan.order[i] = i;
-  }
+  for (int i = 0; i < num; ++i) plan.order[i] = i;
   std::stable_sort(plan.order.begin(), plan.order.end(), [&](int a, int b) {
     return (double)probs[a].n * probs[a].m > (double)probs[b].n * probs[b].m;
   });
@@ -431,6 +606,8 @@ int make_plan(const ottb_problem* probs, int num, int d, const ottb_solver_cfg* 
   }
   plan.off_pristine = off; off = align_up(off + plan.header_bytes);
   plan.total = off;
+  if (need_grid && rows)
+    return plan_rows(plan, d, device_info());
   return OTTB_OK;
 }
 
@@ -495,6 +672,8 @@ int write_header(const ottb_problem* problems, int num_problems, const ottb_solv
     } else {
       P.xt = (const float*)(ws + pp.off_xt);
       P.yt = (const float*)(ws + pp.off_yt);
+      if (pp.keys) P.dkey = (int*)(ws + pp.off_pm + kRowsKeyBytes);
+      if (pp.words) P.words = (unsigned long long*)(ws + pp.off_pm + kRowsSumBytes);
     }
     P.nx = (const float*)(ws + pp.off_nx);
     P.ny = (const float*)(ws + pp.off_ny);
@@ -540,6 +719,10 @@ int write_header(const ottb_problem* problems, int num_problems, const ottb_solv
     ptrs[2 * num_problems + 2 * t] = q.f_init;
     ptrs[2 * num_problems + 2 * t + 1] = q.g_init;
   }
+  if (plan.rows.on) {
+    int* q = std::copy(plan.rows.cluster.begin(), plan.rows.cluster.end(), ids);
+    std::copy(plan.rows.grid.begin(), plan.rows.grid.end(), q);
+  }
   prefix[num_problems] = ug;
   prefix[2 * num_problems + 1] = uf;
   sched->num_active = num_problems;
@@ -552,6 +735,55 @@ int write_header(const ottb_problem* problems, int num_problems, const ottb_solv
   const cudaError_t e = cudaMemcpyAsync(ws + plan.off_pristine, host.data(), plan.header_bytes,
                                         cudaMemcpyHostToDevice, stream);
   return e == cudaSuccess ? OTTB_OK : OTTB_ERR_CUDA;
+}
+
+// The row-owner engine's launches: the clusters' problems, then the grid's.
+int launch_rows(const Plan& plan, const ottb_solver_cfg* cfg, char* ws, cudaStream_t stream) {
+  const RowsPlan& R = plan.rows;
+  RowsArgs ra;
+  std::memset(&ra, 0, sizeof(ra));
+  ra.probs = (ProbDev*)(ws + plan.off_probs);
+  ra.state = (ProbState*)(ws + plan.off_state);
+  ra.sched = (Sched*)(ws + plan.off_sched);
+  ra.gl = (Globals*)(ws + plan.off_globals);
+  ra.cfg = *cfg;
+  const int tmo = cfg->timeout_ms > 0 ? cfg->timeout_ms : 60000;
+  ra.timeout_ns = (uint64_t)tmo * 1000000ull;
+  cudaLaunchConfig_t lc;
+  std::memset(&lc, 0, sizeof(lc));
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  void* kargs[] = {&ra};
+  if (!R.cluster.empty()) {
+    ra.ids = (const int*)(ws + plan.off_ids);
+    ra.count = (int)R.cluster.size();
+    ra.resident = 1;
+    if (cfg->phantom_arrivals > 0)
+      ra.expected = (unsigned)(R.nclusters * R.csize + cfg->phantom_arrivals);
+    lc.gridDim = dim3(R.nclusters * R.csize);
+    lc.blockDim = dim3(R.cthreads);
+    lc.dynamicSmemBytes = R.csmem;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = R.csize;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    if (cudaLaunchKernelExC(&lc, R.kern.cluster, kargs) != cudaSuccess) return OTTB_ERR_CUDA;
+  }
+  if (!R.grid.empty()) {
+    ra.ids = (const int*)(ws + plan.off_ids) + R.cluster.size();
+    ra.count = (int)R.grid.size();
+    ra.resident = R.resident ? 1 : 0;
+    ra.seqwords = R.seqwords ? 1 : 0;
+    ra.expected = (unsigned)R.gsize + (unsigned)std::max(0, cfg->phantom_arrivals);
+    lc.gridDim = dim3(R.gsize);
+    lc.blockDim = dim3(kRowsThreads);
+    lc.dynamicSmemBytes = R.gsmem;
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    if (cudaLaunchKernelExC(&lc, R.kern.grid, kargs) != cudaSuccess) return OTTB_ERR_CUDA;
+  }
+  return OTTB_OK;
 }
 
 // The device side of a solve: restore the header from its pristine copy,
@@ -597,13 +829,21 @@ int launch_solve(int num_problems, int d, const ottb_solver_cfg* cfg, ottb_resul
       prep_points_kernel<<<grid, 256, 0, stream>>>(pa);
   }
   {
-    InitArgs ia{d_ptrs + 2 * num_problems, d_probs, cfg->mask_init};
+    InitArgs ia{d_ptrs + 2 * num_problems, d_probs, cfg->mask_init, plan.rows.on ? 1 : 0};
     dim3 grid((unsigned)std::min<int64_t>((maxpts + 255) / 256, 1024), num_problems);
     init_potentials_kernel<<<grid, 256, 0, stream>>>(ia);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return OTTB_ERR_CUDA;
 
+  if (plan.rows.on) {
+    const int st = launch_rows(plan, cfg, ws, stream);
+    if (st != OTTB_OK || !finalize) return st;
+    FinalArgs fa{d_probs, (ProbState*)(ws + plan.off_state), (Sched*)(ws + plan.off_sched),
+                 results, *cfg};
+    finalize_kernel<<<num_problems, 512, 0, stream>>>(fa);
+    return cuda_status(cudaGetLastError());
+  }
   KernelArgs ka;
   std::memset(&ka, 0, sizeof(ka));
   ka.probs = d_probs;

@@ -1,0 +1,171 @@
+// The FP32 row-owner engine (engine_rows.cuh) as the solve's host side sees
+// it: launch arguments, the split of rows over a team, the shared-memory
+// layout and the kernel table.
+#pragma once
+
+#include "common.cuh"
+
+namespace ottb {
+
+constexpr int kRowsMaxDim = 16;
+constexpr int kRowsThreads = 512;    // most threads of a CTA
+constexpr int kRowsWarps = kRowsThreads / 32;
+constexpr int kRowsMaxCluster = 16;
+constexpr int kRowsMaxCtas = 240;    // most CTAs of a grid team
+constexpr int kRowsChunk = 2048;     // columns per streamed chunk (1024 for D > 10)
+constexpr int kRowsPass = 384;       // most rows of a CTA reduced in one pass over the columns
+constexpr int kRowsOwnFloats = 8192; // most floats of a CTA's own rows kept in shared memory
+constexpr int kRowsKeptRows = 8192;  // most own rows whose last log-sum-exp is kept
+constexpr int kRowsKeyBytes = 3840;  // grid: the shift-change keys, behind the CTAs' sums
+
+struct RowsArgs {
+  ProbDev* probs;
+  ProbState* state;
+  Sched* sched;
+  Globals* gl;
+  const int* ids;       // the launch's problems, table positions
+  int count;
+  int resident;         // grid team: both point sets in shared memory
+  int seqwords;         // grid team: values exchanged as {value, sweep number} words
+  unsigned expected;    // barrier arrivals (CTAs + phantom arrivals; clusters: 0 without phantoms)
+  uint64_t timeout_ns;
+  ottb_solver_cfg cfg;
+};
+
+__host__ __device__ constexpr int rows_chunk(int D) { return D > 10 ? kRowsChunk / 2 : kRowsChunk; }
+
+// First row of team member `rank` of `size`: whole quads of rows.
+__host__ __device__ __forceinline__ int64_t rows_begin(int64_t n, int rank, int size) {
+  const int64_t q = (n + 3) / 4;
+  const int64_t r = 4 * (q * rank / size);
+  return r < n ? r : n;
+}
+
+// Most rows a member of a team of `size` owns of n, rounded up to a quad.
+__host__ __device__ __forceinline__ int64_t rows_most(int64_t n, int size) {
+  const int64_t q = (n + 3) / 4;
+  return 4 * ((q + size - 1) / size);
+}
+
+// Shared-memory layout of a CTA for one problem, offsets in floats (0 where
+// the mode has no such array). Every array starts on 16 bytes.
+//   cluster: points, norms, the exchanged column values of both sides (y
+//     twice, by g parity), the own rows' potentials
+//   grid, resident: points
+//   grid, streamed: two chunks of the column side's points; the own rows'
+//     points where they fit
+// then the own rows' norms, potentials and log-sum-exps, the column shifts,
+// the warps' partial (shift, sum) of the CTA's rows
+// and the own rows' log weights.
+struct RowsLayout {
+  int n4, m4;          // points rounded up to a quad
+  int rf, rg;          // most own rows of the f- and g-sweep (whole quads)
+  int rp;              // rows per pass
+  int own;             // own rows' data in shared memory
+  int cx, cy, nx, ny;  // points [D][n4], [D][m4], norms
+  int ax, ay, anx, any;  // streamed: own rows' points [D][rf], [D][rg], norms
+  int vx, vy;          // cluster: exchanged values [n4 + 4], [2][m4 + 4]
+  int px, py;          // own rows' potentials [rf], [2][rg]
+  int lx, ly;          // own rows' log-sum-exps of their last sweep [rf], [rg] (0: not kept)
+  int wx, wy;          // resident: column shifts of both sides
+  int w, wstride;      // streamed: two chunks' column shifts
+  int pm, pl, logm;
+  int total;
+};
+
+__host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, int size, int warps,
+                                                  bool cluster, bool resident) {
+  RowsLayout L{};
+  L.n4 = (int)((n + 3) / 4 * 4);
+  L.m4 = (int)((m + 3) / 4 * 4);
+  L.rf = (int)rows_most(n, size);
+  L.rg = (int)rows_most(m, size);
+  const int most = L.rf > L.rg ? L.rf : L.rg;
+  L.rp = most < kRowsPass ? most : kRowsPass;
+  L.own = cluster || (int64_t)(L.rf + L.rg) * (D + 1) <= kRowsOwnFloats ? 1 : 0;
+  int64_t p = 0;
+  auto take = [&](int64_t k) {
+    const int64_t o = p;
+    p += (k + 3) / 4 * 4;
+    return (int)o;
+  };
+  if (cluster || resident) {
+    L.cx = take((int64_t)D * L.n4);
+    L.cy = take((int64_t)D * L.m4);
+    if (cluster) {
+      L.nx = take(L.n4);
+      L.ny = take(L.m4);
+    }
+    L.wx = take(L.n4 + 4);
+    L.wy = take(L.m4 + 4);
+    if (cluster) {
+      L.vx = take(L.n4 + 4);
+      L.vy = take(2 * ((int64_t)L.m4 + 4));
+    }
+  } else {
+    L.cx = take(2 * (int64_t)rows_chunk(D) * D);
+    L.wstride = rows_chunk(D) + 4;
+    L.w = take(2 * (int64_t)L.wstride);
+    if (L.own) {
+      L.ax = take((int64_t)D * L.rf);
+      L.ay = take((int64_t)D * L.rg);
+    }
+  }
+  if (!cluster && L.own) {
+    L.anx = take(L.rf);
+    L.any = take(L.rg);
+  }
+  if (L.rf + L.rg <= kRowsKeptRows) {
+    L.lx = take(L.rf);
+    L.ly = take(L.rg);
+  }
+  L.pm = take((int64_t)warps * L.rp);
+  L.pl = take((int64_t)warps * L.rp);
+  if (L.own) {
+    L.px = take(L.rf);
+    L.py = take(2 * (int64_t)L.rg);
+    L.logm = take(2 * ((int64_t)L.rf + L.rg));
+  }
+  L.total = p > (1 << 28) ? 1 << 28 : (int)p;
+  return L;
+}
+
+// What the grid team's CTAs exchange, 8 bytes a point of workspace: column
+// shifts (potentials where the epsilon multiplier varies), x's and two
+// buffers of y's, either plain floats behind the barrier or words {value,
+// sweep number}: a reader polls the data itself, so a new value reaches it
+// in one trip through L2 (write, poll) instead of three (write and release,
+// barrier, load). They live in the region of the tiled engines' split
+// partials, behind the CTAs' error sums, where they fit. What a word held is
+// overwritten only by a CTA that has read every word of the sweep between,
+// and every CTA writes those after it has read the old ones (the g words
+// have two buffers). Every CTA reads every word: measured on B200, a sweep
+// of n = m = 2048, d = 2 takes 12.1 k cycles with words and 13.9 k with the
+// barrier; of n = 7013, m = 5001, d = 3, 56 k with words and 43 k with the
+// barrier (148 CTAs poll 56 KB each). Hence the limit on n + m.
+constexpr int64_t kRowsWordsMax = 6000;
+constexpr size_t kRowsSumBytes = 4096;  // 2 doubles a CTA (up to kRowsMaxCtas), the keys
+__host__ __device__ __forceinline__ size_t rows_words_bytes(int64_t n, int64_t m) {
+  return kRowsSumBytes + 8 * (size_t)(n + 2 * m);
+}
+// Dynamic shared memory of a CTA, in bytes.
+__host__ __device__ inline size_t rows_smem(int64_t n, int64_t m, int D, int size, int warps,
+                                            bool cluster, bool resident) {
+  // beyond any CTA's shared memory (and the offsets' range)
+  if ((cluster || resident) && (n + m) * (int64_t)(D + 1) > (1 << 20)) return (size_t)1 << 30;
+  return (size_t)rows_layout(n, m, D, size, warps, cluster, resident).total * 4;
+}
+
+struct RowsKernel {
+  int D = 0;                      // coordinates the kernel reads (>= d)
+  const void* grid = nullptr;     // one team: the whole grid (cooperative launch)
+  const void* cluster = nullptr;  // teams: thread-block clusters of any size
+};
+
+// The kernels for dimension d; D = 0 above kRowsMaxDim.
+RowsKernel rows_kernel(int d);
+
+// Static shared memory of the kernels, in bytes.
+size_t rows_static_smem();
+
+}  // namespace ottb

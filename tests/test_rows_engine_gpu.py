@@ -1,0 +1,88 @@
+"""The FP32 row-owner engine against the float64 oracle where its split of
+the work changes: single CTAs, clusters and the whole grid, columns resident
+and streamed, several passes over the columns, remainders of quads and
+tiles, every padded dimension, potentials exchanged by words and behind the
+barrier. Tolerances are the FP32 path's (helpers.assert_parity)."""
+import numpy as np
+import pytest
+
+from tests import helpers, problems
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(n, m, d, seed, **kw):
+  x, y, a, b = problems.uniform_cloud_problem(n, m, d, seed=seed)
+  geo = dict(epsilon=0.05, relative_epsilon="mean")
+  geom, out = helpers.gpu_solve(x, y, a, b, precision="fp32", **geo, **kw)
+  ref = helpers.oracle_solve(x, y, a, b, batch_size=1024, **geo, **kw)
+  helpers.assert_parity(geom, out, ref)
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 16])
+@pytest.mark.parametrize("n,m", [(45, 70), (1501, 1303)])
+def test_dimensions(n, m, d):
+  """One CTA or a small cluster; the grid with resident columns."""
+  _check(n, m, d, seed=d)
+
+
+@pytest.mark.parametrize("n,m,d", [
+    (1, 1, 2), (1, 300, 3), (300, 1, 3), (3, 5, 4), (129, 33, 2),   # fewer rows than CTAs
+    (511, 513, 2), (900, 1100, 2),                                  # clusters
+    (2900, 3101, 3), (3007, 2999, 16),        # grid: words; streamed columns
+    (5001, 4003, 2), (2049, 8193, 5),         # grid: the barrier, resident; streamed, a short chunk
+    (60013, 37, 2), (29, 58001, 3),           # several passes; skewed sizes
+])
+def test_sizes(n, m, d):
+  _check(n, m, d, seed=n)
+
+
+@pytest.mark.parametrize("n,m,d", [(60, 45, 3), (700, 400, 2), (2500, 2600, 3), (6001, 5003, 2)])
+def test_epsilon_decay_and_late_blocks(n, m, d):
+  """Multipliers other than 1 (the exchange of potentials instead of
+  shifts), blocks whose error is not asked for, a marginal sweep of its own
+  at the end."""
+  import torch
+  from oracle import sinkhorn_np as oracle
+  from ott_b200.geometry import epsilon_scheduler, pointcloud
+  from ott_b200.solvers import linear
+  x, y, a, b = problems.uniform_cloud_problem(n, m, d, seed=5)
+  for kw in (dict(), dict(min_iterations=25), dict(max_iterations=15, inner_iterations=5,
+                                                   min_iterations=15)):
+    eps = epsilon_scheduler.Epsilon(target=0.02, init=20.0, decay=0.7)
+    geom = pointcloud.PointCloud(torch.as_tensor(x).cuda(), torch.as_tensor(y).cuda(), epsilon=eps)
+    out = linear.solve(geom, torch.as_tensor(a).cuda(), torch.as_tensor(b).cuda(), **kw)
+    ref = oracle.solve(x, y, a, b, epsilon=0.02, eps_init=20.0, eps_decay=0.7, batch_size=1024,
+                       **kw)
+    assert out.n_iters == ref.n_iters
+    helpers.assert_parity(geom, out, ref)
+
+
+def test_batch_of_every_team():
+  """One call whose problems go to clusters and, the large ones, to the
+  grid; the clusters solve several problems one after another."""
+  import torch
+  from ott_b200.geometry import pointcloud
+  from ott_b200.solvers import linear
+  sizes = [(7, 9), (40, 300), (3000, 2500), (129, 128), (1, 4), (600, 601), (64, 5000)] + \
+      [(90 + 7 * k, 210 - 3 * k) for k in range(40)]
+  ps = [problems.uniform_cloud_problem(n, m, 3, seed=i) for i, (n, m) in enumerate(sizes)]
+  cu = lambda t: torch.as_tensor(t).cuda()  # noqa: E731
+  geoms = [pointcloud.PointCloud(cu(p[0]), cu(p[1]), epsilon=0.02) for p in ps]
+  outs = linear.solve_batch(geoms, [cu(p[2]) for p in ps], [cu(p[3]) for p in ps])
+  for p, geom, out in zip(ps, geoms, outs):
+    ref = helpers.oracle_solve(*p, epsilon=0.02, batch_size=1024)
+    helpers.assert_parity(geom, out, ref)
+
+
+def test_zero_weights_of_a_whole_quad():
+  """Rows and columns at -inf, a quad of them at a time."""
+  x, y, a, b = problems.uniform_cloud_problem(1300, 1500, 3, seed=2)
+  a[8:12] = 0
+  b[:5] = 0
+  b[-3:] = 0
+  a, b = (a / a.sum()).astype(np.float32), (b / b.sum()).astype(np.float32)
+  kw = dict(epsilon=0.05, relative_epsilon="mean")
+  geom, out = helpers.gpu_solve(x, y, a, b, **kw)
+  ref = helpers.oracle_solve(x, y, a, b, **kw)
+  helpers.assert_parity(geom, out, ref)
