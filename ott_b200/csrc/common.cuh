@@ -313,6 +313,38 @@ __device__ __forceinline__ void write_ext_row(void* row16, float w) {
   *reinterpret_cast<uint4*>(row16) = v;
 }
 
+// log2 of a positive normal float in FP64: 64 table entries (1 / c_i and
+// log2 c_i for the centres c_i of equal parts of [1, 2)), r = m / c_i - 1
+// with |r| < 2^-7, and the series of log(1 + r) to r^7 (the next term is
+// below 2^-59). A third of the latency of log2(double) and free of
+// branches, so that several rows' evaluations overlap: these stand in every
+// sweep's tail.
+struct Log2Table {
+  double inv[64], lg[64];
+};
+__device__ __forceinline__ void log2_table_fill(Log2Table& t) {
+  for (int i = threadIdx.x; i < 64; i += blockDim.x) {
+    const double inv = 1.0 / (1.0 + (i + 0.5) / 64.0);
+    t.inv[i] = inv;
+    t.lg[i] = -log2(inv);
+  }
+}
+// Whether log2_table takes v (else: log2()).
+__device__ __forceinline__ bool log2_table_ok(float v) { return v > 1e-37f && v < 3e38f; }
+__device__ __forceinline__ double log2_table(const Log2Table& t, float v) {
+  const unsigned b = __float_as_uint(v);
+  const int i = (b >> 17) & 63;
+  const double m = (double)__uint_as_float((b & 0x7fffffu) | 0x3f800000u);
+  const double r = fma(m, t.inv[i], -1.0);
+  const double r2 = r * r;
+  // log(1 + r) / r, by pairs
+  const double p01 = fma(r, -0.5, 1.0);
+  const double p23 = fma(r, -0.25, 1.0 / 3.0);
+  const double p45 = fma(r, -1.0 / 6.0, 0.2);
+  const double p = fma(r2, fma(r2, fma(r2, 1.0 / 7.0, p45), p23), p01);
+  return (double)((int)(b >> 23) - 127) + fma(r * p, kLog2eD, t.lg[i]);
+}
+
 // Merge two (shift, sum) log-sum-exp states in base 2.
 __device__ __forceinline__ void lse_merge(float& m, float& l, float m2, float l2) {
   float mx = fmaxf(m, m2);

@@ -217,35 +217,122 @@ __device__ void finalize_rows_g(const ProbDev& P, const SweepParams& sp, int par
   }
 }
 
-// The same for one warp: lane l holds rows l, l + 32, l + 64, l + 96 of the
-// row block (mv[k], lv[k] for row l + 32 k). Reductions by shuffles only.
-__device__ __forceinline__ void finalize_rows_warp(const ProbDev& P, const SweepParams& sp,
-                                                   int parity, int rb, const float (&mv)[4],
-                                                   const float (&lv)[4], int norm_error) {
+// What the update of a warp's four rows (lane l: rows l + 32 k of the row
+// block) reads that does not depend on the sweep: loaded while the warp
+// waits for the sweep's sums.
+struct RowInputs {
+  float nrm[4], old[4], mg[4];
+  double logm[4];
+};
+
+__device__ __forceinline__ void load_row_inputs(const ProbDev& P, const SweepParams& sp,
+                                                int parity, int rb, const Log2Table& tab,
+                                                RowInputs& in) {
   const int lane = threadIdx.x & 31;
-  const int64_t R = sp.kind == kSweepG ? P.m : P.n;
-  const float ws = sweep_wscale(P, sp.mult);
-  const double eps = update_epsilon(ws);
-  double err = 0.0, msum = 0.0;
-  float dmax = -INFINITY, dmin = INFINITY;
+  const bool isG = sp.kind == kSweepG;
+  const int64_t R = isG ? P.m : P.n;
+  const float* marg = isG ? P.b : P.a;
+  const float* na = isG ? P.ny : P.nx;
+  const float* oldp = isG ? P.gbuf[parity] : P.f;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int64_t r = (int64_t)rb * kBM + lane + 32 * k;
-    if (r < R) {
-      double e, m;
-      finalize_row(P, sp, parity, r, mv[k], lv[k], ws, eps, norm_error, dmax, dmin, e, m);
-      err += e;
-      msum += m;
-    }
+    const bool in_range = r < R;
+    in.nrm[k] = in_range ? na[r] : 0.f;
+    in.mg[k] = in_range ? marg[r] : 1.f;
+    in.old[k] = in_range ? __ldcg(oldp + r) : 0.f;
   }
-  if (sp.write && P.dkey && !P.symmetric) {
-    for (int off = 16; off > 0; off >>= 1) {
-      dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, off));
-      dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, off));
+#pragma unroll
+  for (int k = 0; k < 4; ++k) in.logm[k] = kLn2 * log2_table(tab, in.mg[k]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (!log2_table_ok(in.mg[k])) in.logm[k] = log((double)in.mg[k]);  // 0, subnormal, NaN
+}
+
+// finalize_rows_g for one warp (mv[k], lv[k]: the state of row l + 32 k),
+// the four rows' arithmetic interleaved. A row after the other, each with
+// log2() and log() in FP64 behind its own loads, took ~8000 cycles of a
+// sweep's tail at n = m = 4096.
+__device__ __forceinline__ void finalize_rows_warp(const ProbDev& P, const SweepParams& sp,
+                                                   int parity, int rb, const float (&mv)[4],
+                                                   const float (&lv)[4], int norm_error,
+                                                   const Log2Table& tab, const RowInputs& in) {
+  const int lane = threadIdx.x & 31;
+  const bool isG = sp.kind == kSweepG;
+  const int64_t R = isG ? P.m : P.n;
+  const int64_t r0 = (int64_t)rb * kBM + lane;
+  const float ws = sp.mult == 1.0f ? P.ws_t : sweep_wscale(P, sp.mult);
+  const double eps = update_epsilon(ws);
+  double lse2[4], app[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) lse2[k] = (double)mv[k] + log2_table(tab, lv[k]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (!log2_table_ok(lv[k]))
+      lse2[k] = lv[k] > 0.f ? (double)mv[k] + log2((double)lv[k])
+                            : (lv[k] == 0.f ? -INFINITY : (double)NAN);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) app[k] = eps * kLn2 * lse2[k] - (double)in.nrm[k];
+  if (P.lprev) {
+    float* lp = P.lprev + (isG ? P.n_pad : 0) + r0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (r0 + 32 * k < R) lp[32 * k] = (float)lse2[k];
+  }
+  if (sp.write) {
+    float* outp = (isG ? P.gbuf[parity ^ 1] : P.f) + r0;
+    char* ext = (char*)(isG ? P.exty : P.extx);
+    if (ext) ext += ((isG ? (int64_t)(parity ^ 1) * P.m_pad : 0) + r0) * 16;
+    float dmax = -INFINITY, dmin = INFINITY;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float old = in.old[k];
+      const bool fo = isfinite(old);
+      double newp = eps * in.logm[k] - (fo && isfinite(app[k]) ? app[k] : 0.0);
+      // symmetric problem: Momentum(value=0.5) on the parallel update,
+      // (1 - w) * where(isfinite(old), old, 0) + w * new (acceleration.py:168-170)
+      if (P.symmetric) newp = 0.5 * (fo ? (double)old : 0.0) + 0.5 * newp;
+      const float nf = (float)newp;
+      if (r0 + 32 * k < R) {
+        outp[32 * k] = nf;
+        // the updated point's column shift for the next sweep
+        if (ext) write_ext_row(ext + 32 * 16 * k, (nf - in.nrm[k]) * P.ws_t);
+        if (isfinite(nf) && fo) {
+          const float dl = (nf - old) * P.ws_t;
+          dmax = fmaxf(dmax, dl);
+          dmin = fminf(dmin, dl);
+        } else if (isfinite(nf) != fo) {
+          // a potential became or stopped being -inf: no bound
+          dmax = INFINITY;
+          dmin = -INFINITY;
+        }
+      }
     }
-    if (lane == 0) publish_shift_change(P, sp, dmax, dmin);
+    if (P.dkey && !P.symmetric) {
+      for (int off = 16; off > 0; off >>= 1) {
+        dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, off));
+        dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, off));
+      }
+      if (lane == 0) publish_shift_change(P, sp, dmax, dmin);
+    }
   }
   if (sp.eval) {
+    double err = 0.0, msum = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t r = r0 + 32 * k;
+      if (r < R) {
+        const double mg = (double)in.mg[k];
+        double bh = 0.0;
+        if (!(in.old[k] == -INFINITY))
+          bh = exp2(lse2[k] + ((double)in.old[k] - (double)in.nrm[k]) * (double)ws);
+        const double dv = fabs(bh - mg);
+        err += (norm_error == 1) ? dv : pow(dv, (double)norm_error);
+        msum += bh;
+        if (sp.final_eval && P.marg_out) P.marg_out[r] = (float)bh;
+        if (sp.final_eval && P.lse_out) P.lse_out[r] = (float)app[k];
+      }
+    }
     for (int off = 16; off > 0; off >>= 1) {
       err += __shfl_xor_sync(0xffffffffu, err, off);
       msum += __shfl_xor_sync(0xffffffffu, msum, off);

@@ -382,35 +382,6 @@ __device__ __forceinline__ void cluster_store(uint32_t addr, int v) {
   asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-// log2 of a positive normal float in FP64: 64 table entries (1 / c_i and
-// log2 c_i for the centres c_i of equal parts of [1, 2)), r = m / c_i - 1
-// with |r| < 2^-7, and the series of log(1 + r) to r^7 (the next term is
-// below 2^-59). About a third of log2(double)'s latency, which stood in
-// every sweep's tail.
-struct RowsLog2 {
-  double inv[64], lg[64];
-};
-__device__ __forceinline__ void rows_log2_fill(RowsLog2& t) {
-  for (int i = threadIdx.x; i < 64; i += blockDim.x) {
-    const double inv = 1.0 / (1.0 + (i + 0.5) / 64.0);
-    t.inv[i] = inv;
-    t.lg[i] = -log2(inv);
-  }
-}
-__device__ __forceinline__ double rows_log2(const RowsLog2& t, float v) {
-  const unsigned b = __float_as_uint(v);
-  const int i = (b >> 17) & 63;
-  const double m = (double)__uint_as_float((b & 0x7fffffu) | 0x3f800000u);
-  const double r = fma(m, t.inv[i], -1.0);
-  const double r2 = r * r;
-  // log(1 + r) / r, by pairs
-  const double p01 = fma(r, -0.5, 1.0);
-  const double p23 = fma(r, -0.25, 1.0 / 3.0);
-  const double p45 = fma(r, -1.0 / 6.0, 0.2);
-  const double p = fma(r2, fma(r2, fma(r2, 1.0 / 7.0, p45), p23), p01);
-  return (double)((int)(b >> 23) - 127) + fma(r * p, kLog2eD, t.lg[i]);
-}
-
 // Remote store that signals its bytes on the receiving CTA's mbarrier.
 __device__ __forceinline__ void cluster_store_async(uint32_t addr, float v, uint32_t bar) {
   asm volatile(
@@ -470,7 +441,7 @@ struct RowsShared {
   RowsLayout L;
   GridBarrier bar_grid;
   int rank, size;  // this CTA in its team
-  RowsLog2 log2t;
+  Log2Table log2t;
   RowsCmd cmd[2];
   RowsState st;
   RowsCover cover[2];    // per sweep kind
@@ -978,7 +949,7 @@ struct RowsSolver {
                             : log((double)(isG ? P.b : P.a)[row]);
     if (mx == kNegSentinel && lv < 1.f) lv = 0.f;  // every column at -inf
     double lse2;
-    if (lv > 1e-30f && lv < 3e38f) lse2 = (double)mx + rows_log2(rows_sh.log2t, lv);
+    if (log2_table_ok(lv)) lse2 = (double)mx + log2_table(rows_sh.log2t, lv);
     else lse2 = lv > 0.f ? (double)mx + log2((double)lv)
                          : (lv == 0.f ? -INFINITY : (double)NAN);
     const double app = cmd.epsln2 * lse2 - nrm;
@@ -1267,7 +1238,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) sinkhorn_rows_kernel(RowsArgs
     for (int k = 0; k < 3; ++k) tc::mbar_init(&rows_sh.bar[k], 1);
     tc::fence_barrier_init();
   }
-  rows_log2_fill(rows_sh.log2t);
+  log2_table_fill(rows_sh.log2t);
   __syncthreads();
   // clusters have no grid barrier: a call that asks for phantom arrivals
   // ends here with its timeout

@@ -145,6 +145,7 @@ struct TcSmem {
   uint64_t part_free[2];  // the finalizer has read part buffer b
   uint32_t tmem_base;
   int err;
+  Log2Table log2t;
 };
 
 // Pipeline positions, one copy per thread, advanced identically by every

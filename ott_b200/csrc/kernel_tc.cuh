@@ -94,11 +94,21 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
     const int* ids = sp.final_eval ? A.eval_ids : A.active_ids;
     const int* pre = sp.final_eval ? A.eval_prefix
                                    : (A.prefix + (sp.kind == kSweepG ? 0 : A.num_problems + 1));
-    const int count = sp.final_eval ? ld_sched(&A.sched->num_eval)
-                                    : ld_sched(&A.sched->num_active);
-    const int total = sp.final_eval ? ld_sched(&A.sched->eval_units)
-                                    : ld_sched(&A.sched->total_units[sp.kind == kSweepG ? 0 : 1]);
+    // A call of one problem needs no look at the unit list (a chain of four
+    // trips to L2 before the sweep's first unit): problem 0, its splits.
+    const bool one = A.num_problems == 1;
+    const int count = one ? 1 : sp.final_eval ? ld_sched(&A.sched->num_eval)
+                                              : ld_sched(&A.sched->num_active);
+    const int one_split = one ? split_of(A.state[0], sp.kind) : 0;
+    const int total = one ? (sp.kind == kSweepG      ? A.probs[0].rb_g
+                             : A.probs[0].symmetric ? 0  // f = g
+                                                    : A.probs[0].rb_f) * one_split
+                      : sp.final_eval ? ld_sched(&A.sched->eval_units)
+                                      : ld_sched(&A.sched->total_units[sp.kind == kSweepG ? 0 : 1]);
     const bool dynamic = ld_sched(&A.sched->dynamic_units) != 0;
+    // the bounded row shift of the one problem: its keys' loads are in flight
+    // with the others
+    const RowShift one_shift = one ? bounded_row_shift(A.probs[0], sp) : RowShift{};
     unsigned* ctr = &A.gl->unit_ctr[sweep_idx % 3];
     if (blockIdx.x == 0 && lane == 0) A.gl->unit_ctr[(sweep_idx + 1) % 3] = 0u;
     int rr = blockIdx.x;
@@ -121,12 +131,12 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
         ended = true;
         if (lane == 0) u.end = 1;
       } else {
-        const int q = warp_find_problem(pre, count, ui);
+        const int q = one ? 0 : warp_find_problem(pre, count, ui);
         if (lane == 0) {
-          const int p = __ldcg(ids + q);
+          const int p = one ? 0 : __ldcg(ids + q);
           const ProbDev& P = A.probs[p];
-          const int local = ui - __ldcg(pre + q);
-          const int S = split_of(A.state[p], sp.kind);
+          const int local = one ? ui : ui - __ldcg(pre + q);
+          const int S = one ? one_split : split_of(A.state[p], sp.kind);
           u.end = 0;
           u.p = p;
           u.S = S;
@@ -139,9 +149,9 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
           u.t1 = (int)(((int64_t)ntiles * (u.sidx + 1)) / S);
           // The x layout carries the exponent scale of the target epsilon; a
           // sweep at another epsilon scales the accumulator by ws / ws_t.
-          u.r = sweep_wscale(P, sp.mult) / P.ws_t;
+          u.r = sp.mult == 1.0f ? 1.0f : sweep_wscale(P, sp.mult) / P.ws_t;
           u.op = make_tc_operands(P, sp.kind, u.parity);
-          u.rs = bounded_row_shift(P, sp);
+          u.rs = one ? one_shift : bounded_row_shift(P, sp);
         }
       }
       __syncwarp();
@@ -164,6 +174,10 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
       const bool stop = u.end != 0 || __any_sync(0xffffffffu, *err != 0);
       if (!stop) {
         const uint32_t pb = pp.unit & 1;
+        const ProbDev& P = A.probs[u.p];
+        // what the update reads besides the sums, while they are computed
+        RowInputs in;
+        load_row_inputs(P, sp, u.parity, u.rb, sm.log2t, in);
         ok = __all_sync(0xffffffffu, tc::mbar_wait(&sm.epi_done[pb], (pp.unit >> 1) & 1, tmo));
         ++pp.unit;
         if (!ok) {
@@ -181,7 +195,6 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
         }
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&sm.part_free[pb]);
-        const ProbDev& P = A.probs[u.p];
         const int64_t R = sp.kind == kSweepG ? P.m : P.n;
         const int64_t rbase = (int64_t)u.rb * kBM;
         bool do_final = true;
@@ -205,20 +218,35 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
           do_final = __shfl_sync(0xffffffffu, last, 0) != 0;
           if (do_final) {
             __threadfence();
+            // four splits of the four rows at a time: 32 loads in flight (one
+            // split of one row after the other took S x 4 trips to L2)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              const int64_t row = rbase + lane + 32 * k;
               mv[k] = kNegSentinel;
               lv[k] = 0.f;
-              if (row < R) {
-                for (int j = 0; j < u.S; ++j)
-                  lse_merge(mv[k], lv[k], __ldcg(P.part_m + (int64_t)j * R + row),
-                            __ldcg(P.part_l + (int64_t)j * R + row));
-              }
+            }
+            for (int j0 = 0; j0 < u.S; j0 += 4) {
+              float m2[4][4], l2[4][4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const int64_t row = rbase + lane + 32 * k;
+                  const bool in_range = j0 + j < u.S && row < R;
+                  const int64_t at = (int64_t)(j0 + j) * R + row;
+                  m2[j][k] = in_range ? __ldcg(P.part_m + at) : kNegSentinel;
+                  l2[j][k] = in_range ? __ldcg(P.part_l + at) : 0.f;
+                }
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                  if (j0 + j < u.S) lse_merge(mv[k], lv[k], m2[j][k], l2[j][k]);
             }
           }
         }
-        if (do_final) finalize_rows_warp(P, sp, u.parity, u.rb, mv, lv, A.cfg.norm_error);
+        if (do_final)
+          finalize_rows_warp(P, sp, u.parity, u.rb, mv, lv, A.cfg.norm_error, sm.log2t, in);
       }
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sm.unit_empty[slot]);
@@ -308,6 +336,7 @@ sinkhorn_tc_kernel(KernelArgs A) {
     tc::tmem_alloc(&sm.tmem_base, TcCfg<DK, TN>::kTmemCols);
     tc::tmem_relinquish();
   }
+  log2_table_fill(sm.log2t);
   // Extension blocks: zero everywhere; A's first 3 K columns are ones.
   {
     uint32_t* a32 = reinterpret_cast<uint32_t*>(sm.Aext);
