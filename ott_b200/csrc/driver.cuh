@@ -221,7 +221,7 @@ __device__ void finalize_rows_g(const ProbDev& P, const SweepParams& sp, int par
 // block) reads that does not depend on the sweep: loaded while the warp
 // waits for the sweep's sums.
 struct RowInputs {
-  float nrm[4], old[4], mg[4];
+  float nrm[4], old[4];
   double logm[4];
 };
 
@@ -234,19 +234,29 @@ __device__ __forceinline__ void load_row_inputs(const ProbDev& P, const SweepPar
   const float* marg = isG ? P.b : P.a;
   const float* na = isG ? P.ny : P.nx;
   const float* oldp = isG ? P.gbuf[parity] : P.f;
+  float mg[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int64_t r = (int64_t)rb * kBM + lane + 32 * k;
     const bool in_range = r < R;
     in.nrm[k] = in_range ? na[r] : 0.f;
-    in.mg[k] = in_range ? marg[r] : 1.f;
+    mg[k] = in_range ? marg[r] : 1.f;
     in.old[k] = in_range ? __ldcg(oldp + r) : 0.f;
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) in.logm[k] = kLn2 * log2_table(tab, in.mg[k]);
+  for (int k = 0; k < 4; ++k) in.logm[k] = kLn2 * log2_table(tab, mg[k]);
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    if (!log2_table_ok(in.mg[k])) in.logm[k] = log((double)in.mg[k]);  // 0, subnormal, NaN
+    if (!log2_table_ok(mg[k])) in.logm[k] = log((double)mg[k]);  // 0, subnormal, NaN
+}
+
+// A row's marginal and its error term.
+__device__ __forceinline__ double row_marginal(double lse2, float old, float nrm, float ws) {
+  return old == -INFINITY ? 0.0 : exp2(lse2 + ((double)old - (double)nrm) * (double)ws);
+}
+__device__ __forceinline__ double marginal_term(double bh, float mg, int norm_error) {
+  const double dv = fabs(bh - (double)mg);
+  return norm_error == 1 ? dv : pow(dv, (double)norm_error);
 }
 
 // finalize_rows_g for one warp (mv[k], lv[k]: the state of row l + 32 k),
@@ -322,12 +332,8 @@ __device__ __forceinline__ void finalize_rows_warp(const ProbDev& P, const Sweep
     for (int k = 0; k < 4; ++k) {
       const int64_t r = r0 + 32 * k;
       if (r < R) {
-        const double mg = (double)in.mg[k];
-        double bh = 0.0;
-        if (!(in.old[k] == -INFINITY))
-          bh = exp2(lse2[k] + ((double)in.old[k] - (double)in.nrm[k]) * (double)ws);
-        const double dv = fabs(bh - mg);
-        err += (norm_error == 1) ? dv : pow(dv, (double)norm_error);
+        const double bh = row_marginal(lse2[k], in.old[k], in.nrm[k], ws);
+        err += marginal_term(bh, (isG ? P.b : P.a)[r], norm_error);
         msum += bh;
         if (sp.final_eval && P.marg_out) P.marg_out[r] = (float)bh;
         if (sp.final_eval && P.lse_out) P.lse_out[r] = (float)app[k];

@@ -77,6 +77,9 @@ struct TcCfg {
   static constexpr int kEpiWarp0 = kCtrlWarps;
   static constexpr int kThreads = 32 * (kCtrlWarps + kEpiWarps);
   static constexpr int kDescSlots = 4;    // unit descriptors in flight
+  // problem records kept in shared memory (a record read through an L1 that
+  // every barrier's acquire empties costs the control warps trips to L2)
+  static constexpr int kProbSlots = DK == 64 ? 112 : 4;
   static constexpr uint32_t kIdesc = tc::idesc_bf16_f32(128, kTileN);
   // extension blocks: R rows x 16 bf16, K-major without swizzle: K half 0
   // (elements 0-7) of all rows first, rows 16 B apart (8-row groups 128 B
@@ -146,7 +149,14 @@ struct TcSmem {
   uint32_t tmem_base;
   int err;
   Log2Table log2t;
+  ProbDev probs[TcCfg<DK, TN>::kProbSlots];
 };
+
+static_assert(sizeof(TcSmem<64, 256>) + 1024 <= 227 * 1024 - 64 &&
+                  sizeof(TcSmem<128, 256>) + 1024 <= 227 * 1024 - 64 &&
+                  sizeof(TcSmem<64, 128>) + 1024 <= 227 * 1024 - 64 &&
+                  sizeof(TcSmem<128, 128>) + 1024 <= 227 * 1024 - 64,
+              "a CTA's shared memory");
 
 // Pipeline positions, one copy per thread, advanced identically by every
 // role over the same sequence of tiles, K chunks and units.

@@ -41,23 +41,25 @@ __device__ __forceinline__ TcOperands make_tc_operands(const ProbDev& P, int kin
 // the bound: D = the largest change of a column shift since the rows' last
 // sweep (0 when no potential changed), usable while the spread of those
 // changes stays within kMaxShiftSpread.
-__device__ __forceinline__ RowShift bounded_row_shift(const ProbDev& P, const SweepParams& sp) {
-  RowShift rs{nullptr, 0.f, 0, false};
-  if (!sp.fast || P.symmetric || !P.lprev || !P.dkey) return rs;
+__device__ __forceinline__ bool shift_bound(const ProbDev& P, const SweepParams& sp, float& dmax) {
+  dmax = 0.f;
+  if (!sp.fast || P.symmetric || !P.lprev || !P.dkey) return false;
   const int* slot = P.dkey + ((sp.kind * 2 + sp.rslot) * 2);
   const int kmax = __ldcg(slot), kmin = __ldcg(slot + 1);
-  float dmax = 0.f, spread = 0.f;
+  float spread = 0.f;
   if (kmax != kDkeyEmptyMax) {
-    if (kmin == kDkeyEmptyMin) return rs;
+    if (kmin == kDkeyEmptyMin) return false;
     dmax = fkey_value(kmax);
     spread = dmax - fkey_value(kmin);
   }
-  if (!(spread <= kMaxShiftSpread) || !isfinite(dmax)) return rs;
-  rs.lprev = P.lprev + (sp.kind == kSweepG ? P.n_pad : 0);
-  rs.dmax = dmax;
-  rs.rows = sp.kind == kSweepG ? P.m : P.n;
-  rs.on = true;
-  return rs;
+  return spread <= kMaxShiftSpread && isfinite(dmax);
+}
+
+__device__ __forceinline__ RowShift row_shift_of(const ProbDev& P, const SweepParams& sp, bool on,
+                                                 float dmax) {
+  if (!on) return RowShift{nullptr, 0.f, 0, false};
+  return RowShift{P.lprev + (sp.kind == kSweepG ? P.n_pad : 0), dmax,
+                  sp.kind == kSweepG ? P.m : P.n, true};
 }
 
 // The problem of unit u in a sweep's unit list: the last q with
@@ -88,6 +90,10 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
   const int lane = threadIdx.x & 31;
   const volatile int* err = &sm.err;
   const uint64_t tmo = A.timeout_ns;
+  // every problem's record is in shared memory, or none
+  auto prob = [&](int p) -> const ProbDev& {
+    return A.num_problems <= TcCfg<DK, TN>::kProbSlots ? sm.probs[p] : A.probs[p];
+  };
 
   if (warp == 2) {
     // dealer: every unit of this CTA, then the end marker
@@ -100,15 +106,16 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
     const int count = one ? 1 : sp.final_eval ? ld_sched(&A.sched->num_eval)
                                               : ld_sched(&A.sched->num_active);
     const int one_split = one ? split_of(A.state[0], sp.kind) : 0;
-    const int total = one ? (sp.kind == kSweepG      ? A.probs[0].rb_g
-                             : A.probs[0].symmetric ? 0  // f = g
-                                                    : A.probs[0].rb_f) * one_split
+    const int total = one ? (sp.kind == kSweepG      ? prob(0).rb_g
+                             : prob(0).symmetric ? 0  // f = g
+                                                 : prob(0).rb_f) * one_split
                       : sp.final_eval ? ld_sched(&A.sched->eval_units)
                                       : ld_sched(&A.sched->total_units[sp.kind == kSweepG ? 0 : 1]);
     const bool dynamic = ld_sched(&A.sched->dynamic_units) != 0;
     // the bounded row shift of the one problem: its keys' loads are in flight
     // with the others
-    const RowShift one_shift = one ? bounded_row_shift(A.probs[0], sp) : RowShift{};
+    float dmax = 0.f;
+    bool on = one && shift_bound(prob(0), sp, dmax);
     unsigned* ctr = &A.gl->unit_ctr[sweep_idx % 3];
     if (blockIdx.x == 0 && lane == 0) A.gl->unit_ctr[(sweep_idx + 1) % 3] = 0u;
     int rr = blockIdx.x;
@@ -134,24 +141,26 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
         const int q = one ? 0 : warp_find_problem(pre, count, ui);
         if (lane == 0) {
           const int p = one ? 0 : __ldcg(ids + q);
-          const ProbDev& P = A.probs[p];
+          const ProbDev& P = prob(p);
           const int local = one ? ui : ui - __ldcg(pre + q);
           const int S = one ? one_split : split_of(A.state[p], sp.kind);
           u.end = 0;
           u.p = p;
           u.S = S;
-          u.rb = local / S;
-          u.sidx = local % S;
+          u.rb = (int)((unsigned)local / (unsigned)S);
+          u.sidx = local - u.rb * S;
           u.parity = sp.final_eval ? __ldcg(&A.state[p].final_parity) : sp.parity;
+          // at most 2^24 tiles and 32 splits: 32-bit products and divisions
           const int64_t cols = sp.kind == kSweepG ? P.n : P.m;
-          const int ntiles = (int)((cols + TN - 1) / TN);
-          u.t0 = (int)(((int64_t)ntiles * u.sidx) / S);
-          u.t1 = (int)(((int64_t)ntiles * (u.sidx + 1)) / S);
+          const unsigned ntiles = (unsigned)((cols + TN - 1) / TN);
+          u.t0 = (int)(ntiles * (unsigned)u.sidx / (unsigned)S);
+          u.t1 = (int)(ntiles * (unsigned)(u.sidx + 1) / (unsigned)S);
           // The x layout carries the exponent scale of the target epsilon; a
           // sweep at another epsilon scales the accumulator by ws / ws_t.
           u.r = sp.mult == 1.0f ? 1.0f : sweep_wscale(P, sp.mult) / P.ws_t;
           u.op = make_tc_operands(P, sp.kind, u.parity);
-          u.rs = one ? one_shift : bounded_row_shift(P, sp);
+          if (!one) on = shift_bound(P, sp, dmax);
+          u.rs = row_shift_of(P, sp, on, dmax);
         }
       }
       __syncwarp();
@@ -174,7 +183,7 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
       const bool stop = u.end != 0 || __any_sync(0xffffffffu, *err != 0);
       if (!stop) {
         const uint32_t pb = pp.unit & 1;
-        const ProbDev& P = A.probs[u.p];
+        const ProbDev& P = prob(u.p);
         // what the update reads besides the sums, while they are computed
         RowInputs in;
         load_row_inputs(P, sp, u.parity, u.rb, sm.log2t, in);
@@ -207,28 +216,34 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
               P.part_l[(int64_t)u.sidx * R + row] = lv[k];
             }
           }
-          __threadfence();
+          // the warp's partials, released by lane 0's arrival; the last
+          // arrival acquires the other splits' (a fence on either side of a
+          // relaxed add took ~1500 cycles more)
           __syncwarp();
           int last = 0;
           if (lane == 0) {
-            const int prev = atomicAdd(&P.arrive[u.rb], 1);
+            int prev;
+            asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;"
+                         : "=r"(prev)
+                         : "l"(P.arrive + u.rb)
+                         : "memory");
             last = prev == u.S - 1;
             if (last) atomicExch(&P.arrive[u.rb], 0);
           }
           do_final = __shfl_sync(0xffffffffu, last, 0) != 0;
           if (do_final) {
-            __threadfence();
-            // four splits of the four rows at a time: 32 loads in flight (one
-            // split of one row after the other took S x 4 trips to L2)
+            // two splits of the four rows at a time: 16 loads in flight (one
+            // split of one row after the other took S x 4 trips to L2; four
+            // splits at a time spill)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               mv[k] = kNegSentinel;
               lv[k] = 0.f;
             }
-            for (int j0 = 0; j0 < u.S; j0 += 4) {
-              float m2[4][4], l2[4][4];
+            for (int j0 = 0; j0 < u.S; j0 += 2) {
+              float m2[2][4], l2[2][4];
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
+              for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                   const int64_t row = rbase + lane + 32 * k;
@@ -238,7 +253,7 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
                   l2[j][k] = in_range ? __ldcg(P.part_l + at) : 0.f;
                 }
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
+              for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                   if (j0 + j < u.S) lse_merge(mv[k], lv[k], m2[j][k], l2[j][k]);
@@ -337,6 +352,12 @@ sinkhorn_tc_kernel(KernelArgs A) {
     tc::tmem_relinquish();
   }
   log2_table_fill(sm.log2t);
+  if (A.num_problems <= TcCfg<DK, TN>::kProbSlots) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(A.probs);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(sm.probs);
+    for (int i = threadIdx.x; i < A.num_problems * (int)(sizeof(ProbDev) / 4); i += blockDim.x)
+      dst[i] = src[i];
+  }
   // Extension blocks: zero everywhere; A's first 3 K columns are ones.
   {
     uint32_t* a32 = reinterpret_cast<uint32_t*>(sm.Aext);
