@@ -217,6 +217,10 @@ int choose_split_tc(int rb, int ntiles, int grid) {
   return best;
 }
 
+// Fewest 128 x 256 tiles of a unit that several problems on the tensor cores
+// are split down to.
+constexpr int kBatchUnitTiles = 5;
+
 // Largest column split the workspace is sized for: 32 for a single
 // problem, 8 per problem in calls with several (splits there only grow once
 // problems have converged).
@@ -555,6 +559,14 @@ int make_plan(const ottb_problem* probs, int num, int d, const ottb_solver_cfg* 
   plan.off_maps = off; off = align_up(off + (plan.tc ? sizeof(TcMaps) * num : 0));
   plan.header_bytes = off;
   plan.probs.resize(num);
+  // Several problems on the tensor cores: units of at most about a quarter of
+  // a CTA's share of a sweep, and at least kBatchUnitTiles, so that the CTA
+  // that draws the last unit of the queue does not keep the others waiting.
+  double sweep_tiles = 0.0;
+  for (int i = 0; i < num; ++i)
+    sweep_tiles += (double)((probs[i].n + kBM - 1) / kBM) * ((probs[i].m + kTcPad - 1) / kTcPad);
+  const int unit_tiles = (int)std::max<double>(
+      kBatchUnitTiles, std::min<double>(sweep_tiles / (4.0 * std::max(1, plan.grid)), 1 << 20));
   for (int t = 0; t < num; ++t) {
     const ottb_problem& q = probs[plan.order[t]];
     ProbPlan& pp = plan.probs[t];
@@ -575,8 +587,8 @@ int make_plan(const ottb_problem* probs, int num, int d, const ottb_solver_cfg* 
     };
     auto base = [&](int rb, int64_t pad) {
       const int nt = (int)(pad / tile_n);
-      return plan.tc && num == 1 ? choose_split_tc(rb, nt, plan.grid)
-                                 : choose_split(rb, nt, plan.grid, num);
+      if (plan.tc && num > 1) return std::max(1, (nt + unit_tiles / 2) / unit_tiles);
+      return plan.tc ? choose_split_tc(rb, nt, plan.grid) : choose_split(rb, nt, plan.grid, num);
     };
     pp.split_f = scaled(base(pp.rb_f, pp.m_pad), pp.smax_f);
     pp.split_g = scaled(base(pp.rb_g, pp.n_pad), pp.smax_g);
