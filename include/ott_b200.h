@@ -447,6 +447,23 @@ int32_t ottb_minres_step_next(double* state, int32_t window, const double* v, do
                               double* w_prev, double* x, double* v_next, double* history,
                               int64_t history_len, int64_t s, void* stream);
 
+/* Gradient of reg_ot_cost w.r.t. (x, y, a, b) with the potentials held fixed
+ * (sinkhorn.py:224-277 and :329-335), for a fixed cost scale, from the plan
+ * applied to a column of ones and the coordinates: row_vec [1 + d, n] = P [1,
+ * y], col_vec [1 + d, m] = P^T [1, x]:
+ *   gx_i = scale 2 inv (row_vec_0i x_i - (P y)_i), gy_j likewise,
+ *   ga_i = scale ([a_i > 0](f_i - eps log a_i - eps) + eps sum(b)), gb_j likewise.
+ * FP64 arithmetic; the outputs are float (out_f32 = 1) or double, [n, d],
+ * [m, d], [n], [m], each may be NULL (and then so may what only it reads).
+ * scale: a double on the device, or NULL (1). sums: 2 doubles of device
+ * workspace (only for ga, gb). */
+int32_t ottb_reg_ot_cost_grads(const float* x, const float* y, const float* a, const float* b,
+                               const float* f, const float* g, const float* row_vec,
+                               const float* col_vec, int64_t n, int64_t m, int32_t d,
+                               double epsilon, double inv_scale_cost, const double* scale,
+                               int32_t out_f32, void* gx, void* gy, void* ga, void* gb,
+                               double* sums, void* stream);
+
 /* Human-readable text of a status code. */
 const char* ottb_status_string(int32_t status);
 

@@ -236,6 +236,10 @@ def load() -> ctypes.CDLL:
     lib.ottb_cost_stats_workspace_size.restype = sz
     lib.ottb_cost_stats.argtypes = [vp, vp, i64, i64, i32, ctypes.c_float, i32, vp, vp, sz, vp]
     lib.ottb_cost_stats.restype = i32
+    f64 = ctypes.c_double
+    lib.ottb_reg_ot_cost_grads.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i64, i64, i32, f64, f64,
+                                           vp, i32, vp, vp, vp, vp, vp, vp]
+    lib.ottb_reg_ot_cost_grads.restype = i32
     mlp = ctypes.POINTER(OttbMlp)
     f32 = ctypes.c_float
     lib.ottb_mlp_workspace_size.argtypes = [mlp, i32]

@@ -61,7 +61,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     _nvcc_shared([os.path.join(CSRC, "capi.cu"), os.path.join(CSRC, "noalloc.cu"),
                   os.path.join(CSRC, "mlp.cu"), os.path.join(CSRC, "transport.cu"),
                   os.path.join(CSRC, "transport_tc.cu"), os.path.join(CSRC, "rows.cu"),
-                  os.path.join(CSRC, "krylov.cu")], OUT,
+                  os.path.join(CSRC, "krylov.cu"), os.path.join(CSRC, "grads.cu")], OUT,
                  verbose)
   peaks = os.path.join(CSRC, "peaks", "peaks.cu")
   if force or not up_to_date(PEAKS_OUT, [peaks]):

@@ -266,7 +266,43 @@ class SinkhornOutput(NamedTuple):
     term is 0.
     """
     with torch.no_grad():
+      if self.geom._scale_cost != "mean":
+        return self._fixed_potential_grads((True,) * 4, None, torch.float64)
       return self._reg_ot_cost_grads()
+
+  def _fixed_potential_grads(self, need: Sequence[bool], scale: Optional[torch.Tensor],
+                             dtype: torch.dtype) -> Tuple[Optional[torch.Tensor], ...]:
+    """``reg_ot_cost_grads`` for a fixed cost scale (``ottb_reg_ot_cost_grads``:
+    FP64 arithmetic), the gradients that ``need`` asks for (None for the
+    others) times the 0-dim ``scale``, in ``dtype`` (float32 or float64)."""
+    geom = self.geom
+    n, m = geom.shape
+    x, y = geom.x.detach(), geom.y.detach()
+    dev = x.device
+    a, b, f, g = (_arrays.as_f32(t, dev).detach() for t in (self.a, self.b, self.f, self.g))
+    new = lambda flag, like: torch.empty_like(like, dtype=dtype) if flag else None  # noqa: E731
+    gx, gy, ga, gb = new(need[0], x), new(need[1], y), new(need[2], a), new(need[3], b)
+
+    def applied(pts, axis):
+      ones = torch.ones((1, pts.shape[0]), dtype=torch.float32, device=dev)
+      return self.apply(torch.cat([ones, pts.t()], 0), axis=axis)
+
+    with torch.no_grad():
+      rv = applied(y, 1) if need[0] or (need[1] and self.symmetric) else None  # [1 + d, n]
+      # symmetric solve: f = g and x = y make P symmetric, so the column
+      # application equals the row one
+      cv = rv if self.symmetric else (applied(x, 0) if need[1] else None)
+      if scale is not None:
+        scale = scale.detach().to(device=dev, dtype=torch.float64).contiguous()
+      sums = torch.empty(2, dtype=torch.float64, device=dev) if need[2] or need[3] else None
+      ptr = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+      st = _lib.load().ottb_reg_ot_cost_grads(
+          x.data_ptr(), y.data_ptr(), a.data_ptr(), b.data_ptr(), f.data_ptr(), g.data_ptr(),
+          ptr(rv), ptr(cv), n, m, geom.dim, float(geom.epsilon), float(geom.inv_scale_cost),
+          ptr(scale), 1 if dtype == torch.float32 else 0, ptr(gx), ptr(gy), ptr(ga), ptr(gb),
+          ptr(sums), _arrays.stream_handle())
+      _lib.check(st, "ottb_reg_ot_cost_grads")
+    return gx, gy, ga, gb
 
   def _reg_ot_cost_grads(self):
     geom = self.geom
@@ -372,8 +408,10 @@ class _RegOTCost(torch.autograd.Function):
   @staticmethod
   @torch.autograd.function.once_differentiable
   def backward(ctx, gout):  # pylint: disable=arguments-differ
-    gx, gy, ga, gb = ctx.out.reg_ot_cost_grads()
     need = ctx.needs_input_grad
+    if ctx.out.geom._scale_cost != "mean":
+      return (*ctx.out._fixed_potential_grads(need[:4], gout, torch.float32), None)
+    gx, gy, ga, gb = ctx.out.reg_ot_cost_grads()
     cast = lambda t, i: (gout * t).to(torch.float32) if need[i] else None
     return cast(gx, 0), cast(gy, 1), cast(ga, 2), cast(gb, 3), None
 
