@@ -132,7 +132,7 @@ int32_t ottb_sinkhorn_pointcloud(const ottb_problem* problems,
  *
  * ottb_sinkhorn_launch: the device half, called with the same arguments as
  * the prepare that filled this workspace. Issues stream operations only (a
- * device-to-device copy that restores the header, memsets and kernel
+ * device-to-device copy that restores the header and kernel
  * launches; no host memory and no synchronisation), so it can be captured
  * into a CUDA graph and replayed. Every launch or replay solves again from
  * the current contents of the problems' x, y, a, b, f_init and g_init;

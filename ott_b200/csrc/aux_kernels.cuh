@@ -19,6 +19,10 @@ struct PrepArgs {
   int dp;
 };
 
+// Threads of the centre's CTA: with 1024, d = 64 takes one round of loads a
+// side (256 threads: four).
+constexpr int kCenterThreads = 1024;
+
 // Common centre of the two clouds: the midpoint of the means of strided
 // samples (at most 256 points each) of x and y. C_ij = |x_i - y_j|^2 does
 // not change under a common translation, but the terms of the expanded
@@ -31,9 +35,9 @@ __device__ void sample_center(const float* x, int64_t n, const float* y, int64_t
   // coordinates of one sample row; 16 loads in flight per thread), then
   // thread k adds the groups' sums in a fixed order: the same value on
   // every call. Needs d <= 128 and blockDim.x >= d.
-  __shared__ double part[2][256];
+  __shared__ double part[2][kCenterThreads];
   const int t = threadIdx.x;
-  const int groups = (blockDim.x < 256 ? blockDim.x : 256) / d;
+  const int groups = (blockDim.x < kCenterThreads ? blockDim.x : kCenterThreads) / d;
   const int k = t % d, grp = t / d;
   int64_t ns_side[2];
   for (int side = 0; side < 2; ++side) {
@@ -126,6 +130,10 @@ __global__ void init_potentials_kernel(InitArgs args) {
   // f over n_pad, then g over both g buffers' m_pad rows (padding rows get
   // the -inf column shift of the tensor-core path)
   const int64_t tot = P.n_pad + 2 * P.m_pad;
+  // the split arrivals start at 0
+  const int blocks = max(P.rb_f, P.rb_g);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < blocks; i += gridDim.x * blockDim.x)
+    P.arrive[i] = 0;
   if (args.rows && P.dkey && blockIdx.x == 0 && threadIdx.x < 8)
     P.dkey[threadIdx.x] = (threadIdx.x & 1) ? kDkeyEmptyMin : kDkeyEmptyMax;
   if (args.rows && P.words)
@@ -181,8 +189,35 @@ __device__ __forceinline__ double cta_sum(double v, double* red) {
   return r;
 }
 
+// The potentials' part of the cost, sum over w > 0 of w (pot - eps log w), and
+// sum of w, this thread's share: four points in flight.
+template <class PotFn>
+__device__ __forceinline__ void cost_terms(const float* w, int64_t cnt, double eps,
+                                           const Log2Table& tab, PotFn pot, double& cost,
+                                           double& sum) {
+  for (int64_t i0 = threadIdx.x; i0 < cnt; i0 += 4 * (int64_t)blockDim.x) {
+    float wv[4], pv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t i = i0 + (int64_t)u * blockDim.x;
+      wv[u] = i < cnt ? w[i] : 0.f;
+      pv[u] = i < cnt ? pot(i) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double a = (double)wv[u];
+      sum += a;
+      const double lg = log2_table_ok(wv[u]) ? kLn2 * log2_table(tab, wv[u]) : a > 0.0 ? log(a) : 0.0;
+      if (a > 0.0) cost += a * ((double)pv[u] - eps * lg);
+    }
+  }
+}
+
 __global__ void finalize_kernel(FinalArgs args) {
   __shared__ double red[32];
+  __shared__ Log2Table tab;
+  log2_table_fill(tab);
+  __syncthreads();
   const int p = blockIdx.x;
   const ProbDev& P = args.probs[p];
   const ProbState& S = args.state[p];
@@ -190,21 +225,14 @@ __global__ void finalize_kernel(FinalArgs args) {
   const float* g = P.gbuf[par];
   const double eps = (double)P.eps_target;
   double da = 0.0, db = 0.0, sa = 0.0, sb = 0.0;
-  for (int64_t i = threadIdx.x; i < P.n; i += blockDim.x) {
-    const double a = (double)P.a[i];
-    // a symmetric problem ends with f = g
-    const float fv = P.symmetric ? g[i] : P.f[i];
-    if (P.symmetric) P.f[i] = fv;
-    sa += a;
-    if (a > 0.0) da += a * ((double)fv - eps * log(a));
-  }
-  for (int64_t j = threadIdx.x; j < P.m; j += blockDim.x) {
-    const double b = (double)P.b[j];
-    const float gv = g[j];
-    sb += b;
-    if (b > 0.0) db += b * ((double)gv - eps * log(b));
-    if (par == 1) P.gbuf[0][j] = gv;
-  }
+  // a symmetric problem ends with f = g
+  if (P.symmetric)
+    for (int64_t i = threadIdx.x; i < P.n; i += blockDim.x) P.f[i] = g[i];
+  const float* f = P.symmetric ? g : P.f;
+  cost_terms(P.a, P.n, eps, tab, [&](int64_t i) { return f[i]; }, da, sa);
+  cost_terms(P.b, P.m, eps, tab, [&](int64_t j) { return g[j]; }, db, sb);
+  if (par == 1)
+    for (int64_t j = threadIdx.x; j < P.m; j += blockDim.x) P.gbuf[0][j] = g[j];
   da = cta_sum(da, red);
   db = cta_sum(db, red);
   sa = cta_sum(sa, red);
@@ -245,8 +273,18 @@ __host__ __device__ inline int moments_len(int d, int second) {
   return 3 + 2 * d + (second ? d * d : 0);
 }
 
-__global__ void moments_kernel(const float* pts, int64_t cnt, int d, int second, double* part) {
+// blockIdx.y = point set.
+struct MomentArgs {
+  const float* pts[2];
+  int64_t cnt[2];
+  double* part[2];
+};
+
+__global__ void moments_kernel(MomentArgs args, int d, int second) {
   extern __shared__ double sh[];
+  const float* pts = args.pts[blockIdx.y];
+  const int64_t cnt = args.cnt[blockIdx.y];
+  double* part = args.part[blockIdx.y];
   const int K = moments_len(d, second);
   double* acc = sh;                                // [K] per-CTA accumulators
   float* tile = reinterpret_cast<float*>(sh + K);  // [64][d]
@@ -261,10 +299,15 @@ __global__ void moments_kernel(const float* pts, int64_t cnt, int d, int second,
     for (int idx = threadIdx.x; idx < rows * d; idx += blockDim.x)
       tile[idx] = pts[c0 * d + idx];
     __syncthreads();
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+    // four threads a row (256 threads): a fixed order all the same
+    {
+      const int r = threadIdx.x >> 2;
       double s = 0.0;
-      for (int k = 0; k < d; ++k) s += (double)tile[r * d + k] * tile[r * d + k];
-      nrm[r] = s;
+      if (r < rows)
+        for (int k = threadIdx.x & 3; k < d; k += 4) s += (double)tile[r * d + k] * tile[r * d + k];
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if ((threadIdx.x & 3) == 0 && r < rows) nrm[r] = s;
     }
     __syncthreads();
     for (int e = threadIdx.x; e < K; e += blockDim.x) {
@@ -300,30 +343,39 @@ __global__ void moments_reduce_kernel(const double* px, const double* py, int nb
   const double* src = k < K ? px : py;
   const int e = k < K ? k : k - K;
   double s = 0.0;
+#pragma unroll 8
   for (int b = 0; b < nblk; ++b) s += src[(int64_t)b * K + e];
   mom[k] = s;
 }
 
 // out[0] = mean(C), out[1] = mean(C^2) (when second != 0) from the moments.
+// One CTA; every sum in a fixed order.
 __global__ void cost_stats_final_kernel(const double* mom, int d, int second, double inv,
                                         double* out) {
+  __shared__ double red[32];
   const int K = moments_len(d, second);
   const double* X = mom;
   const double* Y = mom + K;
   const double n = X[0], m = Y[0];
-  const double mnx = X[1] / n, mny = Y[1] / m;
-  double xy = 0.0, nxy = 0.0, xny = 0.0;
-  for (int k = 0; k < d; ++k) {
+  double xy = 0.0, nxy = 0.0, xny = 0.0, tr = 0.0;
+  for (int k = threadIdx.x; k < d; k += blockDim.x) {
     xy += (X[3 + k] / n) * (Y[3 + k] / m);
     nxy += (X[3 + d + k] / n) * (Y[3 + k] / m);
     xny += (X[3 + k] / n) * (Y[3 + d + k] / m);
   }
+  if (second)
+    for (int q = threadIdx.x; q < d * d; q += blockDim.x) {
+      const int k1 = q / d, k2 = q % d;
+      tr += X[3 + 2 * d + k1 * d + k2] * Y[3 + 2 * d + k2 * d + k1];
+    }
+  xy = cta_sum(xy, red);
+  nxy = cta_sum(nxy, red);
+  xny = cta_sum(xny, red);
+  tr = cta_sum(tr, red);
+  if (threadIdx.x) return;
+  const double mnx = X[1] / n, mny = Y[1] / m;
   out[0] = inv * (mnx + mny - 2.0 * xy);
   if (second) {
-    double tr = 0.0;
-    for (int k1 = 0; k1 < d; ++k1)
-      for (int k2 = 0; k2 < d; ++k2)
-        tr += X[3 + 2 * d + k1 * d + k2] * Y[3 + 2 * d + k2 * d + k1];
     tr /= (n * m);
     const double mnx2 = X[2] / n, mny2 = Y[2] / m;
     out[1] = inv * inv *

@@ -799,9 +799,9 @@ int launch_rows(const Plan& plan, const ottb_solver_cfg* cfg, char* ws, cudaStre
 }
 
 // The device side of a solve: restore the header from its pristine copy,
-// clear the split-arrival counters, then fill errors -> prep points -> init
-// potentials -> persistent loop (cooperative) -> finalize. Stream
-// operations only (a device-to-device copy, memsets, kernel launches).
+// then fill errors -> prep points -> init potentials and the split-arrival
+// counters -> persistent loop (cooperative) -> finalize. Stream
+// operations only (a device-to-device copy, kernel launches).
 // finalize = false leaves out finalize_kernel (the result records, the
 // user g copy): for zero-iteration solves whose only output is marg_out or
 // lse_out, written by the persistent kernel itself.
@@ -811,11 +811,6 @@ int launch_solve(int num_problems, int d, const ottb_solver_cfg* cfg, ottb_resul
   e = cudaMemcpyAsync(ws, ws + plan.off_pristine, plan.header_bytes, cudaMemcpyDeviceToDevice,
                       stream);
   if (e != cudaSuccess) return OTTB_ERR_CUDA;
-  for (int t = 0; t < num_problems; ++t) {
-    const ProbPlan& pp = plan.probs[t];
-    e = cudaMemsetAsync(ws + pp.off_arr, 0, sizeof(int) * std::max(pp.rb_f, pp.rb_g), stream);
-    if (e != cudaSuccess) return OTTB_ERR_CUDA;
-  }
   ProbDev* d_probs = (ProbDev*)(ws + plan.off_probs);
   const float* const* d_ptrs = (const float* const*)(ws + plan.off_ptrs);
   int64_t maxpts = 1;
@@ -828,7 +823,7 @@ int launch_solve(int num_problems, int d, const ottb_solver_cfg* cfg, ottb_resul
   {
     PrepArgs pa{d_ptrs, d_probs, d, plan.dp};
     // the common centre once per problem, then the points
-    center_kernel<<<num_problems, 256, 0, stream>>>(pa);
+    center_kernel<<<num_problems, kCenterThreads, 0, stream>>>(pa);
     int64_t mx = 1;
     for (const ProbPlan& pp : plan.probs) mx = std::max(mx, std::max(pp.n_pad, pp.m_pad));
     // one thread per row (FP32 layout) or one warp per row, 8 rows a warp
@@ -853,7 +848,7 @@ int launch_solve(int num_problems, int d, const ottb_solver_cfg* cfg, ottb_resul
     if (st != OTTB_OK || !finalize) return st;
     FinalArgs fa{d_probs, (ProbState*)(ws + plan.off_state), (Sched*)(ws + plan.off_sched),
                  results, *cfg};
-    finalize_kernel<<<num_problems, 512, 0, stream>>>(fa);
+    finalize_kernel<<<num_problems, 1024, 0, stream>>>(fa);
     return cuda_status(cudaGetLastError());
   }
   KernelArgs ka;
@@ -890,7 +885,7 @@ int launch_solve(int num_problems, int d, const ottb_solver_cfg* cfg, ottb_resul
   if (!finalize) return OTTB_OK;
 
   FinalArgs fa{d_probs, ka.state, ka.sched, results, *cfg};
-  finalize_kernel<<<num_problems, 512, 0, stream>>>(fa);
+  finalize_kernel<<<num_problems, 1024, 0, stream>>>(fa);
   return cuda_status(cudaGetLastError());
 }
 
@@ -1382,7 +1377,9 @@ int32_t ottb_cost_stats(const float* x, const float* y, int64_t n, int64_t m, in
   second = second ? 1 : 0;
   const int K = moments_len(d, second);
   const int64_t pts = std::max(n, m);
-  const int nblk = (int)std::min<int64_t>(148, (pts + 255) / 256);
+  // one tile of 64 rows a CTA until every SM has one (256 rows a CTA left
+  // 16 CTAs at 4096 points)
+  const int nblk = (int)std::min<int64_t>(148, (pts + 63) / 64);
   double* px = (double*)workspace;
   double* py = px + (size_t)K * nblk;
   double* mom = (double*)((char*)workspace + align_up(sizeof(double) * moments_len(d, 1) * 2 * 148));
@@ -1395,10 +1392,10 @@ int32_t ottb_cost_stats(const float* x, const float* y, int64_t n, int64_t m, in
                                    sizeof(float) * 64 * 128)) != cudaSuccess)
       return OTTB_ERR_CUDA;
   }
-  moments_kernel<<<nblk, 256, smem, stream>>>(x, n, d, second, px);
-  moments_kernel<<<nblk, 256, smem, stream>>>(y, m, d, second, py);
-  moments_reduce_kernel<<<(2 * K + 255) / 256, 256, 0, stream>>>(px, py, nblk, K, mom);
-  cost_stats_final_kernel<<<1, 1, 0, stream>>>(mom, d, second, (double)inv_scale_cost, out);
+  const MomentArgs ma{{x, y}, {n, m}, {px, py}};
+  moments_kernel<<<dim3(nblk, 2), 256, smem, stream>>>(ma, d, second);
+  moments_reduce_kernel<<<(2 * K + 63) / 64, 64, 0, stream>>>(px, py, nblk, K, mom);
+  cost_stats_final_kernel<<<1, 256, 0, stream>>>(mom, d, second, (double)inv_scale_cost, out);
   return cuda_status(cudaGetLastError());
 }
 
