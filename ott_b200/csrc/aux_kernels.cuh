@@ -237,14 +237,17 @@ __global__ void finalize_kernel(FinalArgs args) {
   db = cta_sum(db, red);
   sa = cta_sum(sa, red);
   sb = cta_sum(sb, red);
-  __syncthreads();
+  // the error log's length and NaNs, all threads (one thread's loop over its
+  // default 200 entries took 6 us)
+  int valid = 0, any_nan = 0;
+  for (int k = threadIdx.x; k < P.outer; k += blockDim.x) {
+    const float e = P.errors[k];
+    valid += e != -1.f;
+    any_nan |= isnan(e);
+  }
+  any_nan = __syncthreads_or(any_nan);
+  valid = (int)cta_sum((double)valid, red);
   if (threadIdx.x == 0) {
-    int valid = 0, any_nan = 0;
-    for (int k = 0; k < P.outer; ++k) {
-      const float e = P.errors[k];
-      if (e != -1.f) ++valid;
-      if (isnan(e)) any_nan = 1;
-    }
     const float last = P.outer > 0 ? P.errors[P.outer - 1] : -1.f;
     ottb_result r;
     r.reg_ot_cost = da + db + eps * (sa * sb - S.msum);
