@@ -27,4 +27,6 @@ def as_f32(arr: Any, dev: Optional[torch.device] = None) -> torch.Tensor:
 
 
 def stream_handle() -> int:
-  return torch.cuda.current_stream().cuda_stream
+  """The current stream of the current device (``torch.cuda.current_stream()
+  .cuda_stream`` without the Python stream object, ~3 us a call)."""
+  return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())

@@ -626,6 +626,8 @@ class _ApplyProduct:
     self._x, self._y = geom.x, geom.y
     self._f = _arrays.as_f32(f, dev).detach().contiguous().clone()
     self._g = _arrays.as_f32(g, dev).detach().contiguous().clone()
+    # the stream that the workspace and both copies belong to
+    self._stream = _arrays.stream_handle()
     self._num_vec = num_vec
     self._rows_in, self._rows_out = (n, m) if axis == 0 else (m, n)
     ws_bytes = _apply_ws_bytes(n, m, geom.dim, num_vec, axis)
@@ -645,9 +647,10 @@ class _ApplyProduct:
                        f"{(self._num_vec, self._rows_in)}")
     out = torch.empty((self._num_vec, self._rows_out), dtype=torch.float32,
                       device=self._ws.device)
-    _keep_until_done(self._ws, self._f, self._g)
-    st = self._lib.ottb_apply_transport_run(self._handle, v2.data_ptr(), out.data_ptr(),
-                                            _arrays.stream_handle())
+    stream = _arrays.stream_handle()
+    if stream != self._stream:  # on their own stream the allocator orders their reuse
+      _keep_until_done(self._ws, self._f, self._g)
+    st = self._lib.ottb_apply_transport_run(self._handle, v2.data_ptr(), out.data_ptr(), stream)
     _lib.check(st, "ottb_apply_transport_run")
     return out
 
