@@ -253,7 +253,7 @@ struct RowsPlan {
   int csize = 1, cthreads = 0, nclusters = 0;
   size_t csmem = 0;
   int gsize = 0;
-  bool resident = false, seqwords = false;
+  bool resident = false, turns = false, seqwords = false;
   size_t gsmem = 0;
 };
 
@@ -461,15 +461,18 @@ int plan_rows(Plan& plan, int d, const DeviceInfo& di) {
   if (!R.grid.empty()) {
     R.gsize = di.sms;
     for (int t : R.grid) R.gsize = std::min(R.gsize, grid_size(plan.probs[t]));
-    size_t res = 0, str = 0;
+    size_t res = 0, turn = 0, str = 0;
     for (int t : R.grid) {
       const ProbPlan& pp = plan.probs[t];
       res = std::max(res, rows_smem(pp.n, pp.m, D, R.gsize, kRowsWarps, false, true));
+      turn = std::max(turn, rows_smem(pp.n, pp.m, D, R.gsize, kRowsWarps, false, true, true));
       str = std::max(str, rows_smem(pp.n, pp.m, D, R.gsize, kRowsWarps, false, false));
     }
-    R.resident = res <= kRowsSmemMax;
+    // where the two sides fit only one at a time, they take turns
+    R.turns = res > kRowsSmemMax && turn <= kRowsSmemMax;
+    R.resident = R.turns || res <= kRowsSmemMax;
     R.seqwords = R.resident;
-    R.gsmem = R.resident ? res : str;
+    R.gsmem = R.turns ? turn : R.resident ? res : str;
     if (R.gsmem > kRowsSmemMax) return OTTB_ERR_UNSUPPORTED;
     for (int t : R.grid) {
       ProbPlan& pp = plan.probs[t];
@@ -786,6 +789,7 @@ int launch_rows(const Plan& plan, const ottb_solver_cfg* cfg, char* ws, cudaStre
     ra.ids = (const int*)(ws + plan.off_ids) + R.cluster.size();
     ra.count = (int)R.grid.size();
     ra.resident = R.resident ? 1 : 0;
+    ra.turns = R.turns ? 1 : 0;
     ra.seqwords = R.seqwords ? 1 : 0;
     ra.expected = (unsigned)R.gsize + (unsigned)std::max(0, cfg->phantom_arrivals);
     lc.gridDim = dim3(R.gsize);

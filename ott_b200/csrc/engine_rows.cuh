@@ -451,7 +451,10 @@ struct RowsShared {
   double slot[2][kRowsMaxCluster];  // cluster: each CTA's error and marginal sums
   double err, msum;
   double eps;       // update_epsilon at multiplier 1
-  uint64_t bar[3];  // cluster: the values of x and of both g buffers have arrived
+  uint64_t bar[3];  // cluster: the values of x and of both g buffers have arrived; in turns,
+                    // bar[0]: the points of pts_side have
+  int pts_side;     // in turns: 0 x, 1 y, -1 neither
+  unsigned pts_loads;  // ... loads so far
   int q;
   int fail;  // a wait ran out
   int key[2][2];  // resident: largest and smallest change of a column shift, by sweep parity
@@ -470,6 +473,7 @@ struct RowsSolver {
   enum { kInitF, kBlock, kG, kF, kFinal, kDone };
 
   static __device__ __forceinline__ bool resident() { return !GRID || rows_sh.A.resident; }
+  static __device__ __forceinline__ bool turns() { return GRID && rows_sh.A.turns; }
   // the epsilon multiplier is 1 throughout: the team exchanges column shifts
   // instead of potentials
   static __device__ __forceinline__ bool constant() {
@@ -484,7 +488,7 @@ struct RowsSolver {
     const int W = blockDim.x >> 5, wsh = 31 - __clz(W);
     const bool res = resident();
     if (threadIdx.x == 0) {
-      rows_sh.L = rows_layout(P.n, P.m, D, rows_sh.size, W, !GRID, res);
+      rows_sh.L = rows_layout(P.n, P.m, D, rows_sh.size, W, !GRID, res, turns());
       rows_sh.eps = update_epsilon(P.ws_t);
     }
     if (threadIdx.x < 2) {
@@ -512,7 +516,7 @@ struct RowsSolver {
           reinterpret_cast<float4*>(rows_mem + dst + (size_t)k * c4)[i] =
               reinterpret_cast<const float4*>(src + k * pad)[i];
     };
-    if (res) {
+    if (res && !turns()) {
       fill(L.cx, P.xt, P.n_pad, L.n4, D);
       fill(L.cy, P.yt, P.m_pad, L.m4, D);
       if (!GRID) {
@@ -524,7 +528,7 @@ struct RowsSolver {
       for (int i = t; i < x1 - x0; i += nt) rows_mem[L.anx + i] = P.nx[x0 + i];
       for (int i = t; i < y1 - y0; i += nt) rows_mem[L.any + i] = P.ny[y0 + i];
     }
-    if (!res && L.own) {
+    if ((!res || turns()) && L.own) {
       // whole quads: the last own quad may reach into the padding
       if (x1 > x0) {
         for (int k = 0; k < D; ++k)
@@ -559,7 +563,41 @@ struct RowsSolver {
       for (int i = t; i < x1 - x0; i += nt) lg[i] = log((double)P.a[x0 + i]);
       for (int i = t; i < y1 - y0; i += nt) lg[L.rf + i] = log((double)P.b[y0 + i]);
     }
+    // what another layout kept in the points' buffer is behind its first load
+    if (turns()) tc::fence_proxy_async_smem();
     __syncthreads();
+  }
+
+  // In turns: brings the points of the columns of a sweep of `kind` into the
+  // buffer, unless they are there (or on their way). By one thread, once no
+  // thread reads the buffer; sweeps wait for it in points_arrived.
+  static __device__ __noinline__ void load_points(int kind) {
+    const ProbDev& P = rows_sh.P;
+    const bool isG = kind == kSweepG;
+    if (rows_sh.pts_side == (isG ? 0 : 1)) return;
+    rows_sh.pts_side = isG ? 0 : 1;
+    ++rows_sh.pts_loads;
+    const int c4 = isG ? rows_sh.L.n4 : rows_sh.L.m4;
+    const float* src = isG ? P.xt : P.yt;
+    const int64_t pad = isG ? P.n_pad : P.m_pad;
+    tc::mbar_arrive_expect_tx(&rows_sh.bar[0], 4u * (unsigned)(D * c4));
+    // each CTA starts at another coordinate (see columns)
+    int k = rows_sh.rank % D;
+    for (int i = 0; i < D; ++i) {
+      tc::bulk_load(rows_mem + rows_sh.L.cx + k * c4, src + k * pad, 4u * (unsigned)c4,
+                    &rows_sh.bar[0]);
+      k = k + 1 < D ? k + 1 : 0;
+    }
+  }
+  // Waits for the last load's points (also when nobody reads them: a CTA
+  // does not leave while one is in flight).
+  static __device__ __forceinline__ void points_arrived() {
+    const unsigned loads = rows_sh.pts_loads;
+    if (loads == 0) return;
+    if (!tc::mbar_wait(&rows_sh.bar[0], (loads - 1) & 1, rows_sh.A.timeout_ns)) {
+      grid_abort(rows_sh.A.gl, &rows_sh.A.sched->status);
+      rows_sh.fail = 1;
+    }
   }
 
   // persistent_main's loop (fixed_point_loop.py:23-93) as a step between
@@ -619,6 +657,7 @@ struct RowsSolver {
       const unsigned phases = S.phases;
       S = RowsState{};
       S.phases = phases;
+      rows_sh.pts_side = -1;
       next = c.init_f_from_g && scan_end > 0 && !P.symmetric ? (int)kInitF : top();
     } else if (S.next == kBlock) {
       next = block(err);
@@ -676,6 +715,7 @@ struct RowsSolver {
     cmd.s = 2.0f * P.inv_scale * cmd.ws;
     cmd.eps = mult == 1.0f ? rows_sh.eps : update_epsilon(cmd.ws);
     cmd.epsln2 = cmd.eps * kLn2;
+    if (turns()) load_points(cmd.kind);
   }
 
   // ------------------------------------------------------------- columns
@@ -833,6 +873,7 @@ struct RowsSolver {
     }
     int* key = rows_sh.key[cmd.seq & 1];
     if (changes) publish_change(key, mx, mn);
+    if (turns()) points_arrived();
     __syncthreads();
     if (threadIdx.x == 0) {
       float dmax = 0.f;
@@ -852,9 +893,12 @@ struct RowsSolver {
                       ? (isG ? L.wx : L.wy)
                       : cmd.colx ? L.vx : L.vy + cmd.parity * (L.m4 + 4);
     const int lp = (isG ? L.ly : L.lx) + p0 - rows_sh.row0[cmd.kind];
+    const bool tn = turns();
+    const int as = tn ? (isG ? L.rg : L.rf) : a4;
+    const int ax = tn ? (isG ? L.ay : L.ax) : isG ? L.cy : L.cx;
     const auto run = [&](auto warp_fn) {
       warp_fn(isG ? L.cx : L.cy, c4, w, (G * warp) >> wsh, (G * (warp + 1)) >> wsh, G,
-              isG ? L.cy : L.cx, nullptr, a4, p0, a4 - 4, (nrows + 3) / 4,
+              ax, nullptr, as, tn ? p0 - rows_sh.row0[cmd.kind] : p0, as - 4, (nrows + 3) / 4,
               rows_sh.cover[cmd.kind], cmd.s, L.pm + warp * L.rp, L.pl + warp * L.rp, true, lp,
               rows_sh.dmax[cmd.kind]);
     };
@@ -1172,6 +1216,10 @@ struct RowsSolver {
         if (GRID && *(volatile int*)&rows_sh.fail) return false;
         const bool last = p0 + rows_sh.L.rp >= rows_sh.row1[cmd.kind];
         if (last && !cmd.eval && control()) advance(cur ^ 1, false, 0.0, 0.0);
+        // an evaluating sweep that already writes is most often followed by
+        // the other side's
+        if (turns() && last && cmd.eval && cmd.write && control())
+          load_points(rows_sh.P.symmetric ? kSweepG : kSweepF);
         update(cur, p0, nrows, err, msum);
         if (last) break;
         p0 += rows_sh.L.rp;
@@ -1235,6 +1283,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) sinkhorn_rows_kernel(RowsArgs
     rows_sh.bar_grid.phase = 0;
     rows_sh.st.phases = 0;
     rows_sh.fail = 0;
+    rows_sh.pts_loads = 0;
     for (int k = 0; k < 3; ++k) tc::mbar_init(&rows_sh.bar[k], 1);
     tc::fence_barrier_init();
   }
@@ -1267,7 +1316,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) sinkhorn_rows_kernel(RowsArgs
       for (int i = threadIdx.x; i < (int)(sizeof(ProbDev) / 4); i += blockDim.x) dst[i] = src[i];
     }
     __syncthreads();
-    if (!Solver::solve(p)) return;
+    const bool ok = Solver::solve(p);
+    if (Solver::turns()) Solver::points_arrived();
+    if (!ok) return;
   }
 }
 

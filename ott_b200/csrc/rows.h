@@ -25,7 +25,8 @@ struct RowsArgs {
   Globals* gl;
   const int* ids;       // the launch's problems, table positions
   int count;
-  int resident;         // grid team: both point sets in shared memory
+  int resident;         // grid team: a sweep's columns are in shared memory at once
+  int turns;            // ... both point sets in one buffer, in turns
   int seqwords;         // grid team: values exchanged as {value, sweep number} words
   unsigned expected;    // barrier arrivals (CTAs + phantom arrivals; clusters: 0 without phantoms)
   uint64_t timeout_ns;
@@ -51,7 +52,8 @@ __host__ __device__ __forceinline__ int64_t rows_most(int64_t n, int size) {
 // the mode has no such array). Every array starts on 16 bytes.
 //   cluster: points, norms, the exchanged column values of both sides (y
 //     twice, by g parity), the own rows' potentials
-//   grid, resident: points
+//   grid, resident: points; in turns: one buffer for either side's points,
+//     the own rows' points
 //   grid, streamed: two chunks of the column side's points; the own rows'
 //     points where they fit
 // then the own rows' norms, potentials and log-sum-exps, the column shifts,
@@ -63,7 +65,7 @@ struct RowsLayout {
   int rp;              // rows per pass
   int own;             // own rows' data in shared memory
   int cx, cy, nx, ny;  // points [D][n4], [D][m4], norms
-  int ax, ay, anx, any;  // streamed: own rows' points [D][rf], [D][rg], norms
+  int ax, ay, anx, any;  // in turns, streamed: own rows' points [D][rf], [D][rg], norms
   int vx, vy;          // cluster: exchanged values [n4 + 4], [2][m4 + 4]
   int px, py;          // own rows' potentials [rf], [2][rg]
   int lx, ly;          // own rows' log-sum-exps of their last sweep [rf], [rg] (0: not kept)
@@ -74,7 +76,8 @@ struct RowsLayout {
 };
 
 __host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, int size, int warps,
-                                                  bool cluster, bool resident) {
+                                                  bool cluster, bool resident,
+                                                  bool turns) {
   RowsLayout L{};
   L.n4 = (int)((n + 3) / 4 * 4);
   L.m4 = (int)((m + 3) / 4 * 4);
@@ -90,8 +93,14 @@ __host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, i
     return (int)o;
   };
   if (cluster || resident) {
-    L.cx = take((int64_t)D * L.n4);
-    L.cy = take((int64_t)D * L.m4);
+    if (turns) {
+      L.cx = L.cy = take((int64_t)D * (L.n4 > L.m4 ? L.n4 : L.m4));
+      L.ax = take((int64_t)D * L.rf);
+      L.ay = take((int64_t)D * L.rg);
+    } else {
+      L.cx = take((int64_t)D * L.n4);
+      L.cy = take((int64_t)D * L.m4);
+    }
     if (cluster) {
       L.nx = take(L.n4);
       L.ny = take(L.m4);
@@ -150,10 +159,12 @@ __host__ __device__ __forceinline__ size_t rows_words_bytes(int64_t n, int64_t m
 }
 // Dynamic shared memory of a CTA, in bytes.
 __host__ __device__ inline size_t rows_smem(int64_t n, int64_t m, int D, int size, int warps,
-                                            bool cluster, bool resident) {
+                                            bool cluster, bool resident, bool turns = false) {
   // beyond any CTA's shared memory (and the offsets' range)
   if ((cluster || resident) && (n + m) * (int64_t)(D + 1) > (1 << 20)) return (size_t)1 << 30;
-  return (size_t)rows_layout(n, m, D, size, warps, cluster, resident).total * 4;
+  const RowsLayout L = rows_layout(n, m, D, size, warps, cluster, resident, turns);
+  if (turns && !L.own) return (size_t)1 << 30;
+  return (size_t)L.total * 4;
 }
 
 struct RowsKernel {

@@ -86,3 +86,45 @@ def test_zero_weights_of_a_whole_quad():
   geom, out = helpers.gpu_solve(x, y, a, b, **kw)
   ref = helpers.oracle_solve(x, y, a, b, **kw)
   helpers.assert_parity(geom, out, ref)
+
+
+@pytest.mark.parametrize("n,m,d", [
+    (2900, 3101, 10), (4099, 2050, 9), (4801, 4700, 10),  # near the buffer's limits
+    (6007, 301, 8), (37, 6201, 8),                        # skewed: few rows, or CTAs without any
+])
+def test_columns_in_turns(n, m, d):
+  """Both sides' points do not fit in shared memory together, either does."""
+  _check(n, m, d, seed=m)
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(min_iterations=25),
+                                dict(max_iterations=15, inner_iterations=5, min_iterations=15)])
+def test_columns_in_turns_order_of_sweeps(kw):
+  """Multipliers other than 1 and blocks that evaluate without an update."""
+  import torch
+  from oracle import sinkhorn_np as oracle
+  from ott_b200.geometry import epsilon_scheduler, pointcloud
+  from ott_b200.solvers import linear
+  x, y, a, b = problems.uniform_cloud_problem(3100, 3302, 9, seed=5)
+  eps = epsilon_scheduler.Epsilon(target=0.05, init=10.0, decay=0.7)
+  cu = lambda t: torch.as_tensor(t).cuda()  # noqa: E731
+  geom = pointcloud.PointCloud(cu(x), cu(y), epsilon=eps)
+  out = linear.solve(geom, cu(a), cu(b), **kw)
+  ref = oracle.solve(x, y, a, b, epsilon=0.05, eps_init=10.0, eps_decay=0.7, batch_size=1024, **kw)
+  assert out.n_iters == ref.n_iters
+  helpers.assert_parity(geom, out, ref)
+
+
+def test_columns_in_turns_batch():
+  """Several problems of one call through the same buffer."""
+  import torch
+  from ott_b200.geometry import pointcloud
+  from ott_b200.solvers import linear
+  kw = dict(max_iterations=10)
+  ps = [problems.uniform_cloud_problem(n, m, 4, seed=n) for n, m in [(4901, 4902), (4850, 5003)]]
+  cu = lambda t: torch.as_tensor(t).cuda()  # noqa: E731
+  geoms = [pointcloud.PointCloud(cu(p[0]), cu(p[1]), epsilon=0.05) for p in ps]
+  outs = linear.solve_batch(geoms, [cu(p[2]) for p in ps], [cu(p[3]) for p in ps], **kw)
+  for p, geom, out in zip(ps, geoms, outs):
+    ref = helpers.oracle_solve(*p, epsilon=0.05, batch_size=1024, **kw)
+    helpers.assert_parity(geom, out, ref)
