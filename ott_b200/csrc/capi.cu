@@ -332,9 +332,11 @@ int validate_cfg(const ottb_solver_cfg* cfg) {
 // Whether an FP32 call goes to the row-owner engine rather than the tiled
 // one: always at d <= 4, where the tiled engine's loop is bound by its issue
 // slots (n = m = 16000, d = 2: 6.2 against 7.8 ms; n = 7013, m = 5001, d =
-// 3: 5.2 against 11); above, while the points stay in shared memory or, for
-// one problem at d <= 10, also streamed (n = m = 16000, d = 10: 13.3 against
-// 16.8 ms; d = 16: 20.5 against 16.8). A batch goes there when each of its
+// 3: 5.2 against 11); above, while the points stay in shared memory, both
+// sides or in turns (n = m = 3500, d = 12: 1.22 against 2.26 ms; n = 2900, m =
+// 2800, d = 16: 1.37 against 1.48), or, for one problem at d <= 10, also
+// streamed (n = m = 16000, d = 10: 11.9 against 16.8 ms; d = 16: 20.5 against
+// 16.8). A batch goes there when each of its
 // problems fits a cluster of 8 (96 problems up to 4096 points, d = 8, of
 // which a part had to go through the grid one by one: 12.8 against 7.6).
 bool rows_wanted(const ottb_problem* probs, int num, int d) {
@@ -343,7 +345,8 @@ bool rows_wanted(const ottb_problem* probs, int num, int d) {
   if (D <= 4 || (num == 1 && D <= 10)) return true;
   constexpr size_t kFits = 224 * 1024;
   if (num == 1)
-    return rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true) <= kFits;
+    return rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true) <= kFits ||
+           rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true, true) <= kFits;
   for (int i = 0; i < num; ++i)
     if (rows_smem(probs[i].n, probs[i].m, D, 8, kRowsWarps, true, false) > kFits) return false;
   return true;

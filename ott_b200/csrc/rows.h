@@ -35,6 +35,13 @@ struct RowsArgs {
 
 __host__ __device__ constexpr int rows_chunk(int D) { return D > 10 ? kRowsChunk / 2 : kRowsChunk; }
 
+// Column groups (of 4) that a lane takes per iteration: two while their
+// products fit beside the rows' coordinates in registers; one leaves more
+// parts of a CTA's columns, so fewer iterations are padding (n = 3000, m =
+// 4100, d = 10, two against one: 1.34 and 1.19 ms; n = m = 3000, d = 8: 0.95
+// and 0.85; n = 6000, m = 5000, d = 5: 1.51 and 1.54).
+__host__ __device__ constexpr int rows_groups(int D) { return D <= 6 ? 2 : 1; }
+
 // First row of team member `rank` of `size`: whole quads of rows.
 __host__ __device__ __forceinline__ int64_t rows_begin(int64_t n, int rank, int size) {
   const int64_t q = (n + 3) / 4;

@@ -90,6 +90,7 @@ def test_zero_weights_of_a_whole_quad():
 
 @pytest.mark.parametrize("n,m,d", [
     (2900, 3101, 10), (4099, 2050, 9), (4801, 4700, 10),  # near the buffer's limits
+    (2901, 2803, 16), (3503, 2600, 12),
     (6007, 301, 8), (37, 6201, 8),                        # skewed: few rows, or CTAs without any
 ])
 def test_columns_in_turns(n, m, d):
