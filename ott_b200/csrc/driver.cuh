@@ -217,36 +217,37 @@ __device__ void finalize_rows_g(const ProbDev& P, const SweepParams& sp, int par
   }
 }
 
-// What the update of a warp's four rows (lane l: rows l + 32 k of the row
-// block) reads that does not depend on the sweep: loaded while the warp
+// What the update of N rows a lane (lane l: rows row0 + l + 32 k) reads that does not depend on the sweep: loaded while the warp
 // waits for the sweep's sums.
+template <int N>
 struct RowInputs {
-  float nrm[4], old[4];
-  double logm[4];
+  float nrm[N], old[N];
+  double logm[N];
 };
 
+template <int N>
 __device__ __forceinline__ void load_row_inputs(const ProbDev& P, const SweepParams& sp,
-                                                int parity, int rb, const Log2Table& tab,
-                                                RowInputs& in) {
+                                                int parity, int64_t row0, const Log2Table& tab,
+                                                RowInputs<N>& in) {
   const int lane = threadIdx.x & 31;
   const bool isG = sp.kind == kSweepG;
   const int64_t R = isG ? P.m : P.n;
   const float* marg = isG ? P.b : P.a;
   const float* na = isG ? P.ny : P.nx;
   const float* oldp = isG ? P.gbuf[parity] : P.f;
-  float mg[4];
+  float mg[N];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int64_t r = (int64_t)rb * kBM + lane + 32 * k;
+  for (int k = 0; k < N; ++k) {
+    const int64_t r = row0 + lane + 32 * k;
     const bool in_range = r < R;
     in.nrm[k] = in_range ? na[r] : 0.f;
     mg[k] = in_range ? marg[r] : 1.f;
     in.old[k] = in_range ? __ldcg(oldp + r) : 0.f;
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) in.logm[k] = kLn2 * log2_table(tab, mg[k]);
+  for (int k = 0; k < N; ++k) in.logm[k] = kLn2 * log2_table(tab, mg[k]);
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
+  for (int k = 0; k < N; ++k)
     if (!log2_table_ok(mg[k])) in.logm[k] = log((double)mg[k]);  // 0, subnormal, NaN
 }
 
@@ -259,34 +260,38 @@ __device__ __forceinline__ double marginal_term(double bh, float mg, int norm_er
   return norm_error == 1 ? dv : pow(dv, (double)norm_error);
 }
 
-// finalize_rows_g for one warp (mv[k], lv[k]: the state of row l + 32 k),
-// the four rows' arithmetic interleaved. A row after the other, each with
+// finalize_rows_g for one warp (mv[k], lv[k]: the state of row row0 + l
+// + 32 k), N rows a lane with their arithmetic interleaved; an evaluating
+// sweep's error and marginal sums go to the caller. A row after the other, each with
 // log2() and log() in FP64 behind its own loads, took ~8000 cycles of a
 // sweep's tail at n = m = 4096.
+template <int N>
 __device__ __forceinline__ void finalize_rows_warp(const ProbDev& P, const SweepParams& sp,
-                                                   int parity, int rb, const float (&mv)[4],
-                                                   const float (&lv)[4], int norm_error,
-                                                   const Log2Table& tab, const RowInputs& in) {
+                                                   int parity, int64_t row0, const float (&mv)[N],
+                                                   const float (&lv)[N], int norm_error,
+                                                   const Log2Table& tab, const RowInputs<N>& in,
+                                                   double& err, double& msum) {
   const int lane = threadIdx.x & 31;
+  err = msum = 0.0;
   const bool isG = sp.kind == kSweepG;
   const int64_t R = isG ? P.m : P.n;
-  const int64_t r0 = (int64_t)rb * kBM + lane;
+  const int64_t r0 = row0 + lane;
   const float ws = sp.mult == 1.0f ? P.ws_t : sweep_wscale(P, sp.mult);
   const double eps = update_epsilon(ws);
-  double lse2[4], app[4];
+  double lse2[N], app[N];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) lse2[k] = (double)mv[k] + log2_table(tab, lv[k]);
+  for (int k = 0; k < N; ++k) lse2[k] = (double)mv[k] + log2_table(tab, lv[k]);
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
+  for (int k = 0; k < N; ++k)
     if (!log2_table_ok(lv[k]))
       lse2[k] = lv[k] > 0.f ? (double)mv[k] + log2((double)lv[k])
                             : (lv[k] == 0.f ? -INFINITY : (double)NAN);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) app[k] = eps * kLn2 * lse2[k] - (double)in.nrm[k];
+  for (int k = 0; k < N; ++k) app[k] = eps * kLn2 * lse2[k] - (double)in.nrm[k];
   if (P.lprev) {
     float* lp = P.lprev + (isG ? P.n_pad : 0) + r0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < N; ++k)
       if (r0 + 32 * k < R) lp[32 * k] = (float)lse2[k];
   }
   if (sp.write) {
@@ -295,7 +300,7 @@ __device__ __forceinline__ void finalize_rows_warp(const ProbDev& P, const Sweep
     if (ext) ext += ((isG ? (int64_t)(parity ^ 1) * P.m_pad : 0) + r0) * 16;
     float dmax = -INFINITY, dmin = INFINITY;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < N; ++k) {
       const float old = in.old[k];
       const bool fo = isfinite(old);
       double newp = eps * in.logm[k] - (fo && isfinite(app[k]) ? app[k] : 0.0);
@@ -327,25 +332,24 @@ __device__ __forceinline__ void finalize_rows_warp(const ProbDev& P, const Sweep
     }
   }
   if (sp.eval) {
-    double err = 0.0, msum = 0.0;
+    // 32 rows after the other, so that the sums do not depend on N
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < N; ++k) {
       const int64_t r = r0 + 32 * k;
+      double e = 0.0, t = 0.0;
       if (r < R) {
         const double bh = row_marginal(lse2[k], in.old[k], in.nrm[k], ws);
-        err += marginal_term(bh, (isG ? P.b : P.a)[r], norm_error);
-        msum += bh;
+        e = marginal_term(bh, (isG ? P.b : P.a)[r], norm_error);
+        t = bh;
         if (sp.final_eval && P.marg_out) P.marg_out[r] = (float)bh;
         if (sp.final_eval && P.lse_out) P.lse_out[r] = (float)app[k];
       }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-      err += __shfl_xor_sync(0xffffffffu, err, off);
-      msum += __shfl_xor_sync(0xffffffffu, msum, off);
-    }
-    if (lane == 0) {
-      P.err_part[rb] = err;
-      P.msum_part[rb] = msum;
+      for (int off = 16; off > 0; off >>= 1) {
+        e += __shfl_xor_sync(0xffffffffu, e, off);
+        t += __shfl_xor_sync(0xffffffffu, t, off);
+      }
+      err += e;
+      msum += t;
     }
   }
 }

@@ -146,6 +146,9 @@ struct TcSmem {
   uint64_t unit_empty[TcCfg<DK, TN>::kDescSlots];  // producer, MMA and finalizer done with it
   uint64_t epi_done[2];   // the epilogue warps wrote part buffer b
   uint64_t part_free[2];  // the finalizer has read part buffer b
+  uint64_t tail_full;     // once a sweep: `tail` is set
+  double tail_red[4][2];  // the tail's error and marginal sums
+  int tail;  // the CTA's last unit completed its row block, which four epilogue warps finish
   uint32_t tmem_base;
   int err;
   Log2Table log2t;
@@ -169,6 +172,7 @@ struct TcPipe {
   int issued;
   uint32_t desc;   // unit descriptors consumed so far (end markers included)
   uint32_t wdesc;  // dealer: unit descriptors written so far
+  uint32_t sweeps;  // sweeps so far
 };
 
 // Tensor maps of a problem, stored in global memory: the point sets

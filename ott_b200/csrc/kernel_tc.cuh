@@ -9,8 +9,8 @@
 // the next unit's A tile and B tiles and issue its MMAs while the epilogue
 // warps still reduce the current unit's last tiles; the finalizer warp
 // merges, combines and applies each unit's row results while the epilogue
-// warps reduce the next one. Only the sweep's end, a grid barrier, joins
-// all warps.
+// warps reduce the next one (a CTA's last unit: four epilogue warps, a row a
+// lane). Only the sweep's end, a grid barrier, joins all warps.
 #pragma once
 
 #include "engine_tc.cuh"
@@ -95,6 +95,7 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
     return A.num_problems <= TcCfg<DK, TN>::kProbSlots ? sm.probs[p] : A.probs[p];
   };
 
+  int tail_at = -1;  // one warp: its CTA's last unit, if any
   if (warp == 2) {
     // dealer: every unit of this CTA, then the end marker
     const int* ids = sp.final_eval ? A.eval_ids : A.active_ids;
@@ -170,7 +171,11 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
     // finalizer: per unit, merge the column groups' (shift, sum) of each row
     // (lane l: rows l + 32 k), combine the column splits of a row block
     // (the CTA that completes its last split finishes it, as sweep_units)
-    // and update the rows' potentials
+    // and update the rows' potentials. Where the unit is the CTA's last of
+    // the sweep, nothing hides the merge and the update, and the epilogue
+    // warps have nothing left to do: four of them take a row a lane (tail
+    // below).
+    bool handed = false;
     while (true) {
       const uint32_t d = pp.desc++;
       const uint32_t slot = d % NSLOT;
@@ -185,8 +190,8 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
         const uint32_t pb = pp.unit & 1;
         const ProbDev& P = prob(u.p);
         // what the update reads besides the sums, while they are computed
-        RowInputs in;
-        load_row_inputs(P, sp, u.parity, u.rb, sm.log2t, in);
+        RowInputs<4> in;
+        load_row_inputs(P, sp, u.parity, (int64_t)u.rb * kBM, sm.log2t, in);
         ok = __all_sync(0xffffffffu, tc::mbar_wait(&sm.epi_done[pb], (pp.unit >> 1) & 1, tmo));
         ++pp.unit;
         if (!ok) {
@@ -231,41 +236,67 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
             if (last) atomicExch(&P.arrive[u.rb], 0);
           }
           do_final = __shfl_sync(0xffffffffu, last, 0) != 0;
-          if (do_final) {
-            // two splits of the four rows at a time: 16 loads in flight (one
-            // split of one row after the other took S x 4 trips to L2; four
-            // splits at a time spill)
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              mv[k] = kNegSentinel;
-              lv[k] = 0.f;
+        }
+        if (do_final) {
+          // the next descriptor has long been dealt
+          const uint32_t d1 = pp.desc, s1 = d1 % NSLOT;
+          ok = __all_sync(0xffffffffu, tc::mbar_wait(&sm.unit_full[s1], (d1 / NSLOT) & 1, tmo));
+          if (!ok) {
+            if (lane == 0) atomicExch(&sm.err, 1);
+            break;
+          }
+          if (sm.units[s1].end) {
+            handed = true;
+            if (lane == 0) {
+              sm.tail = 1;
+              tc::mbar_arrive(&sm.tail_full);
             }
-            for (int j0 = 0; j0 < u.S; j0 += 2) {
-              float m2[2][4], l2[2][4];
+          } else {
+            if (u.S > 1) {
+              // two splits of the four rows at a time: 16 loads in flight (one
+              // split of one row after the other took S x 4 trips to L2; four
+              // splits at a time spill)
 #pragma unroll
-              for (int j = 0; j < 2; ++j)
+              for (int k = 0; k < 4; ++k) {
+                mv[k] = kNegSentinel;
+                lv[k] = 0.f;
+              }
+              for (int j0 = 0; j0 < u.S; j0 += 2) {
+                float m2[2][4], l2[2][4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const int64_t row = rbase + lane + 32 * k;
-                  const bool in_range = j0 + j < u.S && row < R;
-                  const int64_t at = (int64_t)(j0 + j) * R + row;
-                  m2[j][k] = in_range ? __ldcg(P.part_m + at) : kNegSentinel;
-                  l2[j][k] = in_range ? __ldcg(P.part_l + at) : 0.f;
-                }
+                for (int j = 0; j < 2; ++j)
 #pragma unroll
-              for (int j = 0; j < 2; ++j)
+                  for (int k = 0; k < 4; ++k) {
+                    const int64_t row = rbase + lane + 32 * k;
+                    const bool in_range = j0 + j < u.S && row < R;
+                    const int64_t at = (int64_t)(j0 + j) * R + row;
+                    m2[j][k] = in_range ? __ldcg(P.part_m + at) : kNegSentinel;
+                    l2[j][k] = in_range ? __ldcg(P.part_l + at) : 0.f;
+                  }
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  if (j0 + j < u.S) lse_merge(mv[k], lv[k], m2[j][k], l2[j][k]);
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                  for (int k = 0; k < 4; ++k)
+                    if (j0 + j < u.S) lse_merge(mv[k], lv[k], m2[j][k], l2[j][k]);
+              }
+            }
+            double err_sum, msum;
+            finalize_rows_warp(P, sp, u.parity, rbase, mv, lv, A.cfg.norm_error, sm.log2t, in,
+                               err_sum, msum);
+            if (sp.eval && lane == 0) {
+              P.err_part[u.rb] = err_sum;
+              P.msum_part[u.rb] = msum;
             }
           }
         }
-        if (do_final)
-          finalize_rows_warp(P, sp, u.parity, u.rb, mv, lv, A.cfg.norm_error, sm.log2t, in);
       }
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sm.unit_empty[slot]);
       if (stop) break;
+    }
+    if (!handed && lane == 0) {
+      sm.tail = 0;
+      tc::mbar_arrive(&sm.tail_full);
     }
   } else if (warp < 2) {
     // producer (warp 0) and MMA issuer (warp 1)
@@ -293,6 +324,8 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
   } else {
     // epilogue warps, each on its own: reduce every unit's tiles into the
     // part buffers
+    int at = -1;  // the last unit's slot, which the dealer leaves alone until the next sweep
+    bool ended = false;
     while (true) {
       const uint32_t d = pp.desc++;
       const uint32_t slot = d % NSLOT;
@@ -302,11 +335,78 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
         break;
       }
       const TcUnit& u = sm.units[slot];
-      if (u.end != 0 || __any_sync(0xffffffffu, *err != 0)) break;
+      if (u.end != 0 || __any_sync(0xffffffffu, *err != 0)) {
+        ended = true;
+        break;
+      }
       if (!__all_sync(0xffffffffu, tc_epilogue<DK, TN>(sm, pp, u, tmo))) break;
+      at = (int)slot;
     }
+    // The sweep's tail: the last unit's row block, 32 rows a warp, a row a
+    // lane. By the finalizer warp alone, four rows a lane, the splits' merge
+    // and the update took 7.2k of the 41k cycles of a sweep at n = m = 4096
+    // (d = 64: 1.74 -> 1.59 ms; 96 ragged problems, d = 32: 8.9 -> 8.4).
+    const int q = warp - TcCfg<DK, TN>::kEpiWarp0;
+    if (q < 4 && ended && at >= 0) {
+      const TcUnit& u = sm.units[at];
+      const ProbDev& P = prob(u.p);
+      const int64_t row0 = (int64_t)u.rb * kBM + 32 * q;
+      RowInputs<1> in;
+      load_row_inputs(P, sp, u.parity, row0, sm.log2t, in);
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&sm.tail_full, pp.sweeps & 1, tmo))) {
+        if (lane == 0) atomicExch(&sm.err, 1);
+      } else if (sm.tail) {
+        float mv[1] = {kNegSentinel}, lv[1] = {0.f};
+        if (u.S > 1) {
+          const int64_t R = sp.kind == kSweepG ? P.m : P.n;
+          const int64_t row = row0 + lane;
+          constexpr int U = 8;  // splits in flight
+          for (int j0 = 0; j0 < u.S; j0 += U) {
+            float m2[U], l2[U];
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+              const bool in_range = j0 + j < u.S && row < R;
+              const int64_t a = (int64_t)(j0 + j) * R + row;
+              m2[j] = in_range ? __ldcg(P.part_m + a) : kNegSentinel;
+              l2[j] = in_range ? __ldcg(P.part_l + a) : 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+              if (j0 + j < u.S) lse_merge(mv[0], lv[0], m2[j], l2[j]);
+          }
+        } else {
+          const uint32_t pb = (pp.unit - 1) & 1;
+          const int r = 32 * q + lane;
+          mv[0] = sm.part_m[pb][0][r];
+          lv[0] = sm.part_l[pb][0][r];
+#pragma unroll
+          for (int c = 1; c < CG; ++c)
+            lse_merge(mv[0], lv[0], sm.part_m[pb][c][r], sm.part_l[pb][c][r]);
+        }
+        double err_sum, msum;
+        finalize_rows_warp(P, sp, u.parity, row0, mv, lv, A.cfg.norm_error, sm.log2t, in,
+                           err_sum, msum);
+        if (lane == 0) {
+          sm.tail_red[q][0] = err_sum;
+          sm.tail_red[q][1] = msum;
+        }
+      }
+    }
+    tail_at = q == 0 && ended ? at : -1;
   }
+  ++pp.sweeps;
   __syncthreads();
+  if (tail_at >= 0 && lane == 0 && sp.eval && sm.tail && *err == 0) {
+    const TcUnit& u = sm.units[tail_at];
+    const ProbDev& P = prob(u.p);
+    double e = 0.0, t = 0.0;
+    for (int k = 0; k < 4; ++k) {
+      e += sm.tail_red[k][0];
+      t += sm.tail_red[k][1];
+    }
+    P.err_part[u.rb] = e;
+    P.msum_part[u.rb] = t;
+  }
   return *err == 0;
 }
 
@@ -344,6 +444,7 @@ sinkhorn_tc_kernel(KernelArgs A) {
       tc::mbar_init(&sm.epi_done[i], NE);   // one arrival per epilogue warp
       tc::mbar_init(&sm.part_free[i], 1);   // the finalizer
     }
+    tc::mbar_init(&sm.tail_full, 1);        // the finalizer
     sm.err = 0;
     tc::fence_barrier_init();
   }
@@ -378,7 +479,7 @@ sinkhorn_tc_kernel(KernelArgs A) {
   __syncthreads();
   tc::fence_after_sync();
 
-  TcPipe pp{0u, 0u, 0u, 0u, 0u, 0, 0u, 0u};
+  TcPipe pp{0u, 0u, 0u, 0u, 0u, 0, 0u, 0u, 0u};
   auto sweep = [&](const SweepParams& sp, unsigned idx) -> bool {
     return tc_sweep<DK, TN>(A, sp, idx, sm, pp);
   };
