@@ -200,7 +200,15 @@ int choose_split(int rb, int ntiles, int grid, int num_problems) {
 // and 65536 (4 and 2) and takes fewer, longer units from 2048 to 16384,
 // where more units than one wave cost up to twice the time (n = m = 8192:
 // 2 splits, 3.5 ms to 1e-3, against 6.9 ms with 9).
-int choose_split_tc(int rb, int ntiles, int grid) {
+//
+// 0: no split but equal runs of tiles (kernel_tc.cuh), whose longest is at
+// most one tile above the mean, where that is at least 3 % shorter by the
+// model: a further unit of a run costs about 2 tiles, its pipeline being
+// filled beside the one before. Measured against the splits: n = 10007, m =
+// 7919, d = 50: 1.85 -> 1.73 ms; n = m = 20000, d = 64: 6.4 -> 5.6; n = m =
+// 32768: 15.5 -> 14.7; n = 12001, m = 9003, d = 40, the worst found: 2.14 ->
+// 2.17. runs_max: the most CTAs that may meet in a row block (0: no runs).
+int choose_split_tc(int rb, int ntiles, int grid, int runs_max) {
   if (grid <= 0) return 1;
   int best = 1;
   double best_t = -1.0;
@@ -213,6 +221,14 @@ int choose_split_tc(int rb, int ntiles, int grid) {
       best_t = t;
       best = s;
     }
+  }
+  const int64_t tiles = (int64_t)rb * ntiles, run = tiles / grid;
+  if (run >= 4 && tiles < ((int64_t)1 << 31) / grid) {
+    const double meet = (double)((ntiles + run - 2) / run + 1);
+    const double units = std::ceil((double)run / ntiles) + 1.0;
+    const double t = 4.2 + std::ceil((double)tiles / grid) + 2.0 * (units - 1.0) +
+                     0.33 * meet;
+    if (meet <= runs_max && t < 0.97 * best_t) return 0;
   }
   return best;
 }
@@ -588,16 +604,24 @@ int make_plan(const ottb_problem* probs, int num, int d, const ottb_solver_cfg* 
     const int cap = num > 1 ? kMaxSplitBatch : kMaxSplitSingle;
     pp.smax_f = (int)std::max<int64_t>(1, std::min<int64_t>(cap, pp.m_pad / tile_n));
     pp.smax_g = (int)std::max<int64_t>(1, std::min<int64_t>(cap, pp.n_pad / tile_n));
+    // runs of tiles instead of a split: the default schedule of one problem
+    const bool equal_runs = plan.tc && num == 1 && plan.sched.tile_n == kTcPad &&
+                            plan.sched.split_scale == 4 && !plan.sched.dynamic &&
+                            plan.sched.waves == 0;
     auto scaled = [&](int s0, int smax) {
       return std::max(1, std::min(smax, (s0 * plan.sched.split_scale + 2) / 4));
     };
     auto base = [&](int rb, int64_t pad) {
       const int nt = (int)(pad / tile_n);
       if (plan.tc && num > 1) return std::max(1, (nt + unit_tiles / 2) / unit_tiles);
-      return plan.tc ? choose_split_tc(rb, nt, plan.grid) : choose_split(rb, nt, plan.grid, num);
+      const int runs_max = equal_runs ? std::min(cap, nt) : 0;
+      return plan.tc ? choose_split_tc(rb, nt, plan.grid, runs_max)
+                     : choose_split(rb, nt, plan.grid, num);
     };
-    pp.split_f = scaled(base(pp.rb_f, pp.m_pad), pp.smax_f);
-    pp.split_g = scaled(base(pp.rb_g, pp.n_pad), pp.smax_g);
+    pp.split_f = base(pp.rb_f, pp.m_pad);
+    pp.split_g = base(pp.rb_g, pp.n_pad);
+    if (pp.split_f) pp.split_f = scaled(pp.split_f, pp.smax_f);
+    if (pp.split_g) pp.split_g = scaled(pp.split_g, pp.smax_g);
     const size_t fsz = sizeof(float);
     // FP32 engine: transposed [DP][pad] floats; tensor cores: [2][pad][DK] bf16
     const size_t elt = plan.tc ? 2 * 2 : fsz;

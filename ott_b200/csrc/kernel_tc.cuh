@@ -113,6 +113,20 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
                       : sp.final_eval ? ld_sched(&A.sched->eval_units)
                                       : ld_sched(&A.sched->total_units[sp.kind == kSweepG ? 0 : 1]);
     const bool dynamic = ld_sched(&A.sched->dynamic_units) != 0;
+    // Split 0 (one problem): no units of a split, but the sweep's tiles, row
+    // block after row block, dealt to the CTAs in equal runs. A run's part
+    // of a row block is a unit; S is the number of CTAs whose runs meet it.
+    const bool runs = one && one_split == 0;
+    unsigned tiles = 0, row_tiles = 1, pos = 0, run_end = 0;
+    if (runs) {
+      const ProbDev& P = prob(0);
+      row_tiles = (unsigned)(((sp.kind == kSweepG ? P.n : P.m) + TN - 1) / TN);
+      tiles = row_tiles * (unsigned)(sp.kind == kSweepG ? P.rb_g : P.symmetric ? 0 : P.rb_f);
+      // the host takes runs only where tiles * gridDim.x is below 2^31
+      const unsigned v = tiles * (blockIdx.x + (lane & 1)) / gridDim.x;
+      pos = __shfl_sync(0xffffffffu, v, 0);
+      run_end = __shfl_sync(0xffffffffu, v, 1);
+    }
     // the bounded row shift of the one problem: its keys' loads are in flight
     // with the others
     float dmax = 0.f;
@@ -131,31 +145,49 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
       }
       TcUnit& u = sm.units[slot];
       int ui = 0;
-      if (lane == 0) ui = dynamic ? (int)atomicAdd(ctr, 1u) : rr;
+      if (lane == 0) ui = runs ? 0 : dynamic ? (int)atomicAdd(ctr, 1u) : rr;
       ui = __shfl_sync(0xffffffffu, ui, 0);
       rr += gridDim.x;
       // after an error the end marker lets the other roles unwind at once
-      if (ui >= total || __any_sync(0xffffffffu, *err != 0)) {
+      if ((runs ? pos >= run_end : ui >= total) || __any_sync(0xffffffffu, *err != 0)) {
         ended = true;
         if (lane == 0) u.end = 1;
       } else {
         const int q = one ? 0 : warp_find_problem(pre, count, ui);
+        unsigned rb = 0, first = 0, last = 0, end = 0;
+        if (runs) {
+          rb = pos / row_tiles;
+          end = (rb + 1) * row_tiles;  // of the row block
+          // the CTA of tile t: the last one whose run starts at t or before
+          const unsigned t = (lane & 1) ? end - 1 : end - row_tiles;
+          const unsigned c = ((t + 1) * gridDim.x - 1) / tiles;
+          first = __shfl_sync(0xffffffffu, c, 0);
+          last = __shfl_sync(0xffffffffu, c, 1);
+        }
         if (lane == 0) {
           const int p = one ? 0 : __ldcg(ids + q);
           const ProbDev& P = prob(p);
-          const int local = one ? ui : ui - __ldcg(pre + q);
-          const int S = one ? one_split : split_of(A.state[p], sp.kind);
           u.end = 0;
           u.p = p;
-          u.S = S;
-          u.rb = (int)((unsigned)local / (unsigned)S);
-          u.sidx = local - u.rb * S;
           u.parity = sp.final_eval ? __ldcg(&A.state[p].final_parity) : sp.parity;
-          // at most 2^24 tiles and 32 splits: 32-bit products and divisions
-          const int64_t cols = sp.kind == kSweepG ? P.n : P.m;
-          const unsigned ntiles = (unsigned)((cols + TN - 1) / TN);
-          u.t0 = (int)(ntiles * (unsigned)u.sidx / (unsigned)S);
-          u.t1 = (int)(ntiles * (unsigned)(u.sidx + 1) / (unsigned)S);
+          if (runs) {
+            u.S = (int)(last - first) + 1;
+            u.rb = (int)rb;
+            u.sidx = (int)(blockIdx.x - first);
+            u.t0 = (int)(pos - (end - row_tiles));
+            u.t1 = (int)(min(end, run_end) - (end - row_tiles));
+          } else {
+            const int local = one ? ui : ui - __ldcg(pre + q);
+            const int S = one ? one_split : split_of(A.state[p], sp.kind);
+            u.S = S;
+            u.rb = (int)((unsigned)local / (unsigned)S);
+            u.sidx = local - u.rb * S;
+            // at most 2^24 tiles and 32 splits: 32-bit products and divisions
+            const int64_t cols = sp.kind == kSweepG ? P.n : P.m;
+            const unsigned ntiles = (unsigned)((cols + TN - 1) / TN);
+            u.t0 = (int)(ntiles * (unsigned)u.sidx / (unsigned)S);
+            u.t1 = (int)(ntiles * (unsigned)(u.sidx + 1) / (unsigned)S);
+          }
           // The x layout carries the exponent scale of the target epsilon; a
           // sweep at another epsilon scales the accumulator by ws / ws_t.
           u.r = sp.mult == 1.0f ? 1.0f : sweep_wscale(P, sp.mult) / P.ws_t;
@@ -163,6 +195,7 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
           if (!one) on = shift_bound(P, sp, dmax);
           u.rs = row_shift_of(P, sp, on, dmax);
         }
+        pos = min(end, run_end);
       }
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&sm.unit_full[slot]);
