@@ -101,7 +101,8 @@ struct ProbState {
   int msum_valid;    // msum holds the final state's marginal sum
   int stop_it;       // iteration count at stop
   int split_f;       // column split of this problem's f- and g-sweeps (set
-  int split_g;       // by the host, grown at schedule rebuilds)
+  int split_g;       // by the host, grown at schedule rebuilds; 0, one problem on
+                     // the tensor cores: equal runs of tiles, kernel_tc.cuh)
   double msum;
   // Tensor-core path: order-preserving integer keys (fkey) of the largest
   // and smallest change of the column shifts w_c seen by the next sweep of
