@@ -429,6 +429,8 @@ struct RowsShared {
   RowsCover cover[2];    // per sweep kind
   int iters[2];          // ... and its iterations per warp
   int row0[2], row1[2];  // this CTA's rows, per sweep kind
+  unsigned owners[2];    // cluster, per sweep kind: bit q, CTA q owns rows of it
+  int resync;            // see sums
   double red[2][kRowsWarps];
   double slot[2][kRowsMaxCluster];  // cluster: each CTA's error and marginal sums
   double err, msum;
@@ -465,6 +467,14 @@ struct RowsSolver {
   // rows in small problems
   static __device__ __forceinline__ bool control() { return threadIdx.x == blockDim.x - 1; }
 
+  // Whether this CTA owns rows of a sweep of `kind`. One that owns none (a
+  // side with fewer quads of rows than the team has CTAs) reads none of that
+  // sweep's values and is sent none: whoever reads a sweep's values publishes
+  // in that sweep, on which the exchange without barriers rests (rows.h).
+  static __device__ __forceinline__ bool has_rows(int kind) {
+    return rows_sh.row1[kind] > rows_sh.row0[kind];
+  }
+
   static __device__ __noinline__ void begin() {
     const ProbDev& P = rows_sh.P;
     const int W = blockDim.x >> 5, wsh = 31 - __clz(W);
@@ -489,6 +499,16 @@ struct RowsSolver {
       rows_sh.iters[kind] = rows_iters(rows_sh.cover[kind], (G + W - 1) >> wsh, rows_groups(D));
     }
     if (threadIdx.x < 2) rows_sh.bound[threadIdx.x] = 0;
+    if (threadIdx.x < 32) {
+      const int q = threadIdx.x, size = rows_sh.size;
+      for (int kind = 0; kind < 2; ++kind) {
+        const int64_t rows = kind == kSweepG ? P.m : P.n;
+        const unsigned mask = __ballot_sync(
+            0xffffffffu, q < size && rows_begin(rows, q, size) < rows_begin(rows, q + 1, size));
+        if (q == 0) rows_sh.owners[kind] = mask;
+      }
+      if (q == 0) rows_sh.resync = (min(P.n, P.m) + 3) / 4 < size;
+    }
     const int x0 = rows_sh.row0[kSweepF], x1 = rows_sh.row1[kSweepF];
     const int y0 = rows_sh.row0[kSweepG], y1 = rows_sh.row1[kSweepG];
     const int t = threadIdx.x, nt = blockDim.x;
@@ -690,7 +710,9 @@ struct RowsSolver {
     if (cmd.write) {
       const int to = isf ? 0 : 1 + (cmd.parity ^ 1);
       S.seq_of[to] = cmd.seq;
-      if (!GRID && rows_sh.size > 1) S.pending |= 1u << to;
+      // x's values are read by g-sweeps, y's by f-sweeps (in a symmetric
+      // problem, where every CTA owns the same rows of both, by g-sweeps)
+      if (!GRID && rows_sh.size > 1 && has_rows(isf ? kSweepG : kSweepF)) S.pending |= 1u << to;
     }
     cmd.mult = mult;
     cmd.ws = mult == 1.0f ? P.ws_t : sweep_wscale(P, mult);
@@ -1004,8 +1026,9 @@ struct RowsSolver {
           if (lead) *dst = x;
         } else {
           const uint64_t* b = &rows_sh.bar[isG ? 1 + (parity ^ 1) : 0];
+          const unsigned readers = rows_sh.owners[isG ? kSweepF : kSweepG];
           for (int q = k; q < rows_sh.size; q += lanes)
-            cluster_store_async(cluster_addr(dst, q), x, cluster_addr(b, q));
+            if (readers >> q & 1) cluster_store_async(cluster_addr(dst, q), x, cluster_addr(b, q));
         }
       }
       if (lead && L.own) rows_mem[(isG ? L.py + (parity ^ 1) * L.rg : L.px) + own] = nf;
@@ -1094,6 +1117,9 @@ struct RowsSolver {
 
   // The team's error and marginal sums, in a fixed order (lanes, warps,
   // CTAs), into rows_sh.err and rows_sh.msum of every CTA. False after a timeout.
+  // A CTA without rows waits for nobody's values and may reach the next
+  // evaluating sweep while another still reads this one's sums: a team with
+  // such CTAs meets once more behind the reading (resync).
   static __device__ __noinline__ bool sums(double err, double msum) {
     const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int off = 16; off > 0; off >>= 1) {
@@ -1137,6 +1163,7 @@ struct RowsSolver {
         rows_sh.msum = u;
       }
     }
+    if (rows_sh.resync) return barrier();
     __syncthreads();
     return true;
   }
@@ -1162,8 +1189,12 @@ struct RowsSolver {
       while (true) {
         const int nrows = min(rows_sh.row1[cmd.kind] - p0, rows_sh.L.rp);
         if (resident()) {
-          if (p0 == rows_sh.row0[cmd.kind]) columns(cur);
-          if (nrows > 0) reduce_resident(cur, p0, nrows);
+          if (nrows > 0) {
+            if (p0 == rows_sh.row0[cmd.kind]) columns(cur);
+            reduce_resident(cur, p0, nrows);
+          } else if (turns()) {
+            points_arrived();  // before the next load into the buffer
+          }
         } else {
           const int C = (int)(cmd.kind == kSweepG ? rows_sh.P.n : rows_sh.P.m);
           const int nch = chunks(C);

@@ -154,11 +154,15 @@ __host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, i
 // barrier, load). They live in the region of the tiled engines' split
 // partials, behind the CTAs' error sums, where they fit. What a word held is
 // overwritten only by a CTA that has read every word of the sweep between,
-// and every CTA writes those after it has read the old ones (the g words
-// have two buffers). Every CTA reads every word: measured on B200, a sweep
-// of n = m = 2048, d = 2 takes 12.1 k cycles with words and 13.9 k with the
-// barrier; of n = 7013, m = 5001, d = 3, 56 k with words and 43 k with the
-// barrier (148 CTAs poll 56 KB each). Hence the limit on n + m.
+// and every CTA that reads the old ones writes those after it has read them
+// (the g words have two buffers). A CTA without rows of a sweep therefore
+// reads none of its values: with n = 4000, m = 200 on 148 CTAs, 98 own no
+// row of y and publish nothing in g-sweeps, so nothing would hold back the
+// f-sweep that overwrites what they read. Every CTA with rows reads every
+// word: measured on B200, a sweep of n = m = 2048, d = 2 takes 12.1 k cycles
+// with words and 13.9 k with the barrier; of n = 7013, m = 5001, d = 3, 56 k
+// with words and 43 k with the barrier (148 CTAs poll 56 KB each). Hence the
+// limit on n + m.
 constexpr int64_t kRowsWordsMax = 6000;
 constexpr size_t kRowsSumBytes = 4096;  // 2 doubles a CTA (up to kRowsMaxCtas), the keys
 __host__ __device__ __forceinline__ size_t rows_words_bytes(int64_t n, int64_t m) {

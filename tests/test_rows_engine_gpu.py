@@ -129,3 +129,27 @@ def test_columns_in_turns_batch():
   for p, geom, out in zip(ps, geoms, outs):
     ref = helpers.oracle_solve(*p, epsilon=0.05, batch_size=1024, **kw)
     helpers.assert_parity(geom, out, ref)
+
+
+@pytest.mark.parametrize("inner", [1, 10])
+@pytest.mark.parametrize("n,m", [(4000, 200), (200, 4000), (1000, 40), (4000, 8), (8, 4000), (9, 5)])
+def test_team_members_without_rows(n, m, inner):
+  """CTAs of a grid or cluster that own rows of one side only, or of none:
+  they take no part in the other side's exchange and meet the others in the
+  evaluating sweeps."""
+  _check(n, m, 2, seed=n + m, inner_iterations=inner)
+
+
+def test_batch_with_members_without_rows():
+  """Clusters that draw problems with fewer quads of rows than CTAs between
+  larger ones."""
+  import torch
+  from ott_b200.geometry import pointcloud
+  from ott_b200.solvers import linear
+  sizes = [(1500, 1400), (1300, 9), (7, 1200), (5, 6), (900, 30), (1, 1), (1100, 1000)]
+  ps = [problems.uniform_cloud_problem(n, m, 3, seed=i) for i, (n, m) in enumerate(sizes)]
+  cu = lambda t: torch.as_tensor(t).cuda()  # noqa: E731
+  geoms = [pointcloud.PointCloud(cu(p[0]), cu(p[1]), epsilon=0.05) for p in ps]
+  outs = linear.solve_batch(geoms, [cu(p[2]) for p in ps], [cu(p[3]) for p in ps])
+  for p, geom, out in zip(ps, geoms, outs):
+    helpers.assert_parity(geom, out, helpers.oracle_solve(*p, epsilon=0.05, batch_size=1024))
