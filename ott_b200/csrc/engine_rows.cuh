@@ -702,10 +702,13 @@ struct RowsSolver {
     rows_sh.key[cmd.seq & 1][0] = kDkeyEmptyMax;
     rows_sh.key[cmd.seq & 1][1] = kDkeyEmptyMin;
     if (GRID && P.dkey && rows_sh.rank == 0) {
-      // this sweep's keys: those of the sweep four before it, whose readers
-      // (the sweep after that one) have all passed a barrier since
-      P.dkey[2 * (cmd.seq & 3)] = kDkeyEmptyMax;
-      P.dkey[2 * (cmd.seq & 3) + 1] = kDkeyEmptyMin;
+      // the next sweep's keys (the first one's are clear from the start): its
+      // writers come behind the barrier that ends this sweep, before which
+      // this is written. They were the keys of the sweep three before this
+      // one, whose readers, in the sweep after it, have passed a barrier
+      // since.
+      P.dkey[2 * ((cmd.seq + 1) & 3)] = kDkeyEmptyMax;
+      P.dkey[2 * ((cmd.seq + 1) & 3) + 1] = kDkeyEmptyMin;
     }
     if (cmd.write) {
       const int to = isf ? 0 : 1 + (cmd.parity ^ 1);

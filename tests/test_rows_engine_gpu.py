@@ -153,3 +153,10 @@ def test_batch_with_members_without_rows():
   outs = linear.solve_batch(geoms, [cu(p[2]) for p in ps], [cu(p[3]) for p in ps])
   for p, geom, out in zip(ps, geoms, outs):
     helpers.assert_parity(geom, out, helpers.oracle_solve(*p, epsilon=0.05, batch_size=1024))
+
+
+@pytest.mark.parametrize("inner,its", [(1, 7), (3, 12)])
+def test_streamed_bound_across_evaluating_sweeps(inner, its):
+  """The streamed sweeps' bound on the change of the column shifts, with an
+  evaluating sweep before every update and before some."""
+  _check(6001, 5003, 10, seed=3, inner_iterations=inner, max_iterations=its)
