@@ -507,7 +507,9 @@ struct RowsSolver {
             0xffffffffu, q < size && rows_begin(rows, q, size) < rows_begin(rows, q + 1, size));
         if (q == 0) rows_sh.owners[kind] = mask;
       }
-      if (q == 0) rows_sh.resync = (min(P.n, P.m) + 3) / 4 < size;
+      if (q == 0)
+        rows_sh.resync = (min(P.n, P.m) + 3) / 4 < size ||
+                         (P.symmetric && rows_sh.A.cfg.inner_iterations == 1);
     }
     const int x0 = rows_sh.row0[kSweepF], x1 = rows_sh.row1[kSweepF];
     const int y0 = rows_sh.row0[kSweepG], y1 = rows_sh.row1[kSweepG];
@@ -1120,9 +1122,12 @@ struct RowsSolver {
 
   // The team's error and marginal sums, in a fixed order (lanes, warps,
   // CTAs), into rows_sh.err and rows_sh.msum of every CTA. False after a timeout.
-  // A CTA without rows waits for nobody's values and may reach the next
-  // evaluating sweep while another still reads this one's sums: a team with
-  // such CTAs meets once more behind the reading (resync).
+  // A CTA overwrites its sums in the next evaluating sweep, which must not
+  // begin while another still reads these. Most often the values exchanged in
+  // between see to that. They do not where a CTA without rows waits for
+  // nobody's, nor where every sweep evaluates (blocks of one iteration of a
+  // symmetric problem: the values are out before the sums are read). Such
+  // teams meet once more behind the reading (resync).
   static __device__ __noinline__ bool sums(double err, double msum) {
     const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int off = 16; off > 0; off >>= 1) {

@@ -160,3 +160,33 @@ def test_streamed_bound_across_evaluating_sweeps(inner, its):
   """The streamed sweeps' bound on the change of the column shifts, with an
   evaluating sweep before every update and before some."""
   _check(6001, 5003, 10, seed=3, inner_iterations=inner, max_iterations=its)
+
+
+def _check_symmetric(n, d, eps, init=None, **kw):
+  """The parallel, momentum-1/2 update on x = y, a = b."""
+  import torch
+  from oracle import sinkhorn_np as oracle
+  from ott_b200.geometry import pointcloud
+  from ott_b200.problems.linear import linear_problem
+  from ott_b200.solvers.linear import acceleration, sinkhorn
+  x, _, a, _ = problems.uniform_cloud_problem(n, n, d, seed=n)
+  xt, at = torch.as_tensor(x).cuda(), torch.as_tensor(a).cuda()
+  geom = pointcloud.PointCloud(xt, xt, epsilon=eps)
+  solver = sinkhorn.Sinkhorn(parallel_dual_updates=True, precision="fp32",
+                             momentum=acceleration.Momentum(start=0, value=0.5), **kw)
+  x64, a64 = x.astype(np.float64), a.astype(np.float64)
+  start = {}
+  if init is not None:
+    start["init"] = (init, init)
+  out = solver(linear_problem.LinearProblem(geom, at, at),
+               init=None if init is None else (torch.as_tensor(init).cuda(),) * 2)
+  ref = helpers.oracle_sinkhorn(oracle.Geom(x64, x64, eps, batch_size=1024), a64, a64,
+                                parallel_dual_updates=True, momentum=0.5, **start, **kw)
+  helpers.assert_parity(geom, out, ref)
+
+
+@pytest.mark.parametrize("n", [30, 700, 2501, 5002])
+def test_symmetric_blocks_of_one_iteration(n):
+  """Every sweep evaluates; nothing is exchanged between two sums but the
+  sums themselves."""
+  _check_symmetric(n, 2, 0.05, inner_iterations=1, max_iterations=15)
