@@ -699,7 +699,9 @@ struct RowsSolver {
       S.phases ^= 1u << k;
     }
     cmd.seq = ++S.seq;
-    cmd.change = mult != 1.0f || S.last[cmd.kind] == 0 ? -1 : cmd.want > S.last[cmd.kind] ? 1 : 0;
+    // In a symmetric problem the kind's last sweep has itself written the
+    // columns of this one (want == last).
+    cmd.change = mult != 1.0f || S.last[cmd.kind] == 0 ? -1 : cmd.want >= S.last[cmd.kind] ? 1 : 0;
     S.last[cmd.kind] = mult == 1.0f ? cmd.seq : 0;
     rows_sh.key[cmd.seq & 1][0] = kDkeyEmptyMax;
     rows_sh.key[cmd.seq & 1][1] = kDkeyEmptyMin;

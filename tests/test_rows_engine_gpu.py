@@ -162,7 +162,7 @@ def test_streamed_bound_across_evaluating_sweeps(inner, its):
   _check(6001, 5003, 10, seed=3, inner_iterations=inner, max_iterations=its)
 
 
-def _check_symmetric(n, d, eps, init=None, **kw):
+def _check_symmetric(n, d, eps, **kw):
   """The parallel, momentum-1/2 update on x = y, a = b."""
   import torch
   from oracle import sinkhorn_np as oracle
@@ -175,13 +175,9 @@ def _check_symmetric(n, d, eps, init=None, **kw):
   solver = sinkhorn.Sinkhorn(parallel_dual_updates=True, precision="fp32",
                              momentum=acceleration.Momentum(start=0, value=0.5), **kw)
   x64, a64 = x.astype(np.float64), a.astype(np.float64)
-  start = {}
-  if init is not None:
-    start["init"] = (init, init)
-  out = solver(linear_problem.LinearProblem(geom, at, at),
-               init=None if init is None else (torch.as_tensor(init).cuda(),) * 2)
+  out = solver(linear_problem.LinearProblem(geom, at, at))
   ref = helpers.oracle_sinkhorn(oracle.Geom(x64, x64, eps, batch_size=1024), a64, a64,
-                                parallel_dual_updates=True, momentum=0.5, **start, **kw)
+                                parallel_dual_updates=True, momentum=0.5, **kw)
   helpers.assert_parity(geom, out, ref)
 
 
@@ -190,3 +186,32 @@ def test_symmetric_blocks_of_one_iteration(n):
   """Every sweep evaluates; nothing is exchanged between two sums but the
   sums themselves."""
   _check_symmetric(n, 2, 0.05, inner_iterations=1, max_iterations=15)
+
+
+@pytest.mark.parametrize("n,d,eps", [(1102, 2, 0.004), (2303, 3, 0.003), (5901, 10, 0.02)])
+def test_symmetric_from_given_potentials(n, d, eps):
+  """A warm start from 100 times the epsilon, whose first updates move the
+  column shifts by hundreds of log2 units: clusters, the grid's resident and
+  streamed columns. Ten iterations leave an error at the level of the FP32
+  exponents' rounding (the largest |f - |x|^2| / eps is 150 to 600, times
+  2^-24: 1e-5 to 4e-5 of a row's mass), so what is compared is the potentials,
+  within the FP32 path's 1e-4 eps."""
+  import torch
+  from oracle import sinkhorn_np as oracle
+  from ott_b200.geometry import pointcloud
+  from ott_b200.problems.linear import linear_problem
+  from ott_b200.solvers.linear import acceleration, sinkhorn
+  x, _, a, _ = problems.uniform_cloud_problem(n, n, d, seed=n)
+  x64, a64 = x.astype(np.float64), a.astype(np.float64)
+  kw = dict(min_iterations=10, max_iterations=10, parallel_dual_updates=True)
+  warm = oracle.sinkhorn(oracle.Geom(x64, x64, 100 * eps, batch_size=1024), a64, a64,
+                         momentum=0.5, **kw).f.astype(np.float32)
+  xt, at, wt = (torch.as_tensor(t).cuda() for t in (x, a, warm))
+  solver = sinkhorn.Sinkhorn(momentum=acceleration.Momentum(start=0, value=0.5),
+                             precision="fp32", **kw)
+  geom = pointcloud.PointCloud(xt, xt, epsilon=eps)
+  out = solver(linear_problem.LinearProblem(geom, at, at), init=(wt, wt))
+  ref = oracle.sinkhorn(oracle.Geom(x64, x64, eps, batch_size=1024), a64, a64, momentum=0.5,
+                        init=(warm, warm), **kw)
+  helpers.assert_potentials(out.f.cpu().numpy().astype(np.float64),
+                            out.g.cpu().numpy().astype(np.float64), ref, 1e-4)
