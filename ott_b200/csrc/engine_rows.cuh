@@ -117,9 +117,11 @@ __device__ inline int rows_iters(RowsCover c, int gseg, int NG) {
 }
 
 // The bounded shift of a row: every exponent of the row is at most this. A
-// row without a finite log-sum-exp has no finite term either.
+// row without a finite log-sum-exp has no finite term either; one at -inf
+// gets the running maximum's mark of a row without a term, by which
+// update_row knows it (exp2_poly2 turns its terms into 2^-126, not 0).
 __device__ __forceinline__ float row_sigma(float lprev, float dmax) {
-  return isfinite(lprev) ? lprev + dmax : 0.f;
+  return isfinite(lprev) ? lprev + dmax : lprev == -INFINITY ? kNegSentinel : 0.f;
 }
 
 // One warp's share of a sweep over the columns in shared memory: rows

@@ -215,3 +215,18 @@ def test_symmetric_from_given_potentials(n, d, eps):
                         init=(warm, warm), **kw)
   helpers.assert_potentials(out.f.cpu().numpy().astype(np.float64),
                             out.g.cpu().numpy().astype(np.float64), ref, 1e-4)
+
+
+@pytest.mark.parametrize("n,m,d", [(1000, 1100, 2), (2048, 2000, 3), (2050, 2040, 5), (30001, 700, 3)])
+def test_side_without_weight(n, m, d):
+  """Every column of the other side's sweeps at -inf: a row's log-sum-exp is
+  -inf under the running maximum and under the bounded shift, with part of
+  the exponentials on the polynomial (d <= 3) and without."""
+  x, y, _, b = problems.uniform_cloud_problem(n, m, d, seed=2)
+  kw = dict(epsilon=0.05, max_iterations=20)
+  _, out = helpers.gpu_solve(x, y, np.zeros(n, np.float32), b, precision="fp32", **kw)
+  ref = helpers.oracle_solve(x, y, np.zeros(n), b, batch_size=1024, **kw)
+  helpers.assert_potentials(out.f.cpu().numpy().astype(np.float64),
+                            out.g.cpu().numpy().astype(np.float64), ref, 1e-4)
+  # every marginal is 0: the error is the other side's mass
+  np.testing.assert_allclose(out.errors.cpu().numpy(), ref.errors, rtol=1e-5)
