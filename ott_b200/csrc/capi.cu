@@ -359,18 +359,14 @@ bool rows_wanted(const ottb_problem* probs, int num, int d) {
   const int D = rows_kernel(d).D;
   if (D == 0) return false;
   if (D <= 4 || (num == 1 && D <= 10)) return true;
-  constexpr size_t kFits = 224 * 1024;
+  auto fits = [](size_t bytes) { return bytes <= (size_t)kRowsSmemMax; };
   if (num == 1)
-    return rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true) <= kFits ||
-           rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true, true) <= kFits;
+    return fits(rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true)) ||
+           fits(rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true, true));
   for (int i = 0; i < num; ++i)
-    if (rows_smem(probs[i].n, probs[i].m, D, 8, kRowsWarps, true, false) > kFits) return false;
+    if (!fits(rows_smem(probs[i].n, probs[i].m, D, 8, kRowsWarps, true, false))) return false;
   return true;
 }
-
-// Dynamic shared memory a row-owner CTA may ask for (227 KB less its static
-// part).
-const size_t kRowsSmemMax = 227 * 1024 - rows_static_smem() - 64;
 
 // Clusters of `size` CTAs that the device holds at once. Cached: the query
 // stays out of later calls, which may be under stream capture.

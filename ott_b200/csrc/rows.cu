@@ -32,6 +32,8 @@ RowsKernel rows_kernel(int d) {
   return RowsKernel{};
 }
 
+static_assert(sizeof(RowsShared) + 64 + kRowsSmemMax <= 227 * 1024, "a CTA's shared memory");
+
 size_t rows_static_smem() { return sizeof(RowsShared); }
 
 }  // namespace ottb

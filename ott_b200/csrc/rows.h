@@ -17,6 +17,9 @@ constexpr int kRowsPass = 384;       // most rows of a CTA reduced in one pass o
 constexpr int kRowsOwnFloats = 8192; // most floats of a CTA's own rows kept in shared memory
 constexpr int kRowsKeptRows = 8192;  // most own rows whose last log-sum-exp is kept
 constexpr int kRowsKeyBytes = 3840;  // grid: the shift-change keys, behind the CTAs' sums
+// Dynamic shared memory a CTA may ask for: 227 KB less the kernels' static
+// part (rows.cu checks that it is below 3 KB).
+constexpr int kRowsSmemMax = 224 * 1024;
 
 struct RowsArgs {
   ProbDev* probs;
@@ -66,6 +69,11 @@ __host__ __device__ __forceinline__ int64_t rows_most(int64_t n, int size) {
 // then the own rows' norms, potentials and log-sum-exps, the column shifts,
 // the warps' partial (shift, sum) of the CTA's rows
 // and the own rows' log weights.
+//
+// A streamed layout fits kRowsSmemMax at every size: where it would not (D >=
+// 7: two chunks take 128 or 160 KB), the own rows' data stay in global
+// memory, and passes have at most kRowsPass / 2, then kRowsPass / 4 rows
+// (`cut` 1 to 3).
 struct RowsLayout {
   int n4, m4;          // points rounded up to a quad
   int rf, rg;          // most own rows of the f- and g-sweep (whole quads)
@@ -82,17 +90,18 @@ struct RowsLayout {
   int total;
 };
 
-__host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, int size, int warps,
-                                                  bool cluster, bool resident,
-                                                  bool turns) {
+__host__ __device__ inline RowsLayout rows_layout_cut(int64_t n, int64_t m, int D, int size,
+                                                      int warps, bool cluster, bool resident,
+                                                      bool turns, int cut) {
   RowsLayout L{};
   L.n4 = (int)((n + 3) / 4 * 4);
   L.m4 = (int)((m + 3) / 4 * 4);
   L.rf = (int)rows_most(n, size);
   L.rg = (int)rows_most(m, size);
   const int most = L.rf > L.rg ? L.rf : L.rg;
-  L.rp = most < kRowsPass ? most : kRowsPass;
-  L.own = cluster || (int64_t)(L.rf + L.rg) * (D + 1) <= kRowsOwnFloats ? 1 : 0;
+  const int pass = cut < 2 ? kRowsPass : kRowsPass >> (cut - 1);
+  L.rp = most < pass ? most : pass;
+  L.own = cluster || (cut == 0 && (int64_t)(L.rf + L.rg) * (D + 1) <= kRowsOwnFloats) ? 1 : 0;
   int64_t p = 0;
   auto take = [&](int64_t k) {
     const int64_t o = p;
@@ -143,6 +152,15 @@ __host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, i
     L.logm = take(2 * ((int64_t)L.rf + L.rg));
   }
   L.total = p > (1 << 28) ? 1 << 28 : (int)p;
+  return L;
+}
+
+__host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, int size, int warps,
+                                                  bool cluster, bool resident, bool turns) {
+  int cut = 0;
+  RowsLayout L = rows_layout_cut(n, m, D, size, warps, cluster, resident, turns, cut);
+  while (!cluster && !resident && cut < 3 && L.total > kRowsSmemMax / 4)
+    L = rows_layout_cut(n, m, D, size, warps, cluster, resident, turns, ++cut);
   return L;
 }
 

@@ -230,3 +230,41 @@ def test_side_without_weight(n, m, d):
                             out.g.cpu().numpy().astype(np.float64), ref, 1e-4)
   # every marginal is 0: the error is the other side's mass
   np.testing.assert_allclose(out.errors.cpu().numpy(), ref.errors, rtol=1e-5)
+
+
+def _sinkhorn64(x, y, a, b, eps, iterations):
+  """The float64 iteration in plain torch, for sizes that take numpy minutes:
+  potentials and the last error (of the g marginal)."""
+  import torch
+
+  def lse(p, q, pot):  # eps log sum_j exp((pot_j - C_ij) / eps), rows of p
+    out = torch.empty(p.shape[0], dtype=torch.float64, device=p.device)
+    for i in range(0, p.shape[0], 1024):
+      c = (p[i:i + 1024] ** 2).sum(1, keepdim=True) + (q ** 2).sum(1) - 2.0 * p[i:i + 1024] @ q.T
+      out[i:i + 1024] = eps * torch.logsumexp((pot - c) / eps, dim=1)
+    return out
+
+  x, y, a, b = (torch.as_tensor(t).cuda().double() for t in (x, y, a, b))
+  f, g = torch.zeros_like(a), torch.zeros_like(b)
+  for _ in range(iterations):
+    g = eps * b.log() - lse(y, x, f)
+    f = eps * a.log() - lse(x, y, g)
+  err = (torch.exp((lse(y, x, f) + g) / eps) - b).abs().sum()
+  return f, g, float(err)
+
+
+@pytest.mark.parametrize("n,m,d", [
+    (30000, 30000, 10), (65536, 65536, 8), (500, 40000, 10), (51700, 51600, 7),  # own rows not kept
+    (700001, 100, 9), (950001, 100, 10), (2001, 600001, 10),                     # shorter passes
+])
+def test_large_streamed_dimensions(n, m, d):
+  """Two chunks of d = 7 ... 10 leave little of a CTA's shared memory for
+  the rest of its layout."""
+  x, y, a, b = problems.uniform_cloud_problem(n, m, d, seed=n + d)
+  eps, its = 0.05, 3
+  _, out = helpers.gpu_solve(x, y, a, b, precision="fp32", epsilon=eps, min_iterations=its,
+                             max_iterations=its, inner_iterations=its)
+  f, g, err = _sinkhorn64(x, y, a, b, eps, its)
+  np.testing.assert_allclose(out.f.cpu().numpy(), f.cpu().numpy(), rtol=0, atol=1e-4 * eps)
+  np.testing.assert_allclose(out.g.cpu().numpy(), g.cpu().numpy(), rtol=0, atol=1e-4 * eps)
+  np.testing.assert_allclose(float(out.errors[0]), err, rtol=1e-2, atol=1e-6)
