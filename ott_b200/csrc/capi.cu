@@ -20,6 +20,7 @@
 #include <cuda.h>
 
 #include "aux_kernels.cuh"
+#include "fp32_route.h"
 #include "kernel_simt.cuh"
 #include "kernel_tc.cuh"
 #include "launch.cuh"
@@ -64,7 +65,7 @@ int simt_dp(int d) {
   return dp;
 }
 
-// Kernel table for the tiled CUDA-core engine (d > 4; see rows_wanted).
+// Kernel table for the tiled CUDA-core engine (rows_wanted says when).
 template <int DP>
 struct SimtKernel {
   static void* fn() { return (void*)&sinkhorn_simt_kernel<DP>; }
@@ -80,6 +81,8 @@ struct KernelChoice {
 KernelChoice pick_simt(int dp) {
   KernelChoice k;
   switch (dp) {
+    case 2: k.fn = SimtKernel<2>::fn(); k.smem = SimtKernel<2>::smem(); break;
+    case 4: k.fn = SimtKernel<4>::fn(); k.smem = SimtKernel<4>::smem(); break;
     case 8: k.fn = SimtKernel<8>::fn(); k.smem = SimtKernel<8>::smem(); break;
     case 16: k.fn = SimtKernel<16>::fn(); k.smem = SimtKernel<16>::smem(); break;
     case 32: k.fn = SimtKernel<32>::fn(); k.smem = SimtKernel<32>::smem(); break;
@@ -168,26 +171,6 @@ struct Schedule {
   int dynamic = 0;
   int tile_n = 256;  // tensor-core tile width (256 or 128); the CUDA-core engine ignores it
 };
-
-// Column splits of one sweep: enough units to keep every CTA busy with
-// little tail (efficiency = units / (waves * grid)).
-int choose_split(int rb, int ntiles, int grid, int num_problems) {
-  if (num_problems > 1 || grid <= 0) return 1;
-  int best = 1;
-  double best_score = -1.0;
-  const int smax = std::max(1, std::min(ntiles, 32));
-  for (int s = 1; s <= smax; ++s) {
-    const double units = (double)rb * s;
-    const double waves = std::ceil(units / grid);
-    const double eff = units / (waves * grid);
-    const double score = eff - 0.004 * s;
-    if (score > best_score + 1e-9) {
-      best_score = score;
-      best = s;
-    }
-  }
-  return best;
-}
 
 // Column splits of a single problem on the tensor cores: the split that
 // minimises a cost model of one sweep, in units of one 128 x 256 tile's
@@ -345,29 +328,6 @@ int validate_cfg(const ottb_solver_cfg* cfg) {
   return OTTB_OK;
 }
 
-// Whether an FP32 call goes to the row-owner engine rather than the tiled
-// one: always at d <= 4, where the tiled engine's loop is bound by its issue
-// slots (n = m = 16000, d = 2: 6.2 against 7.8 ms; n = 7013, m = 5001, d =
-// 3: 5.2 against 11); above, while the points stay in shared memory, both
-// sides or in turns (n = m = 3500, d = 12: 1.22 against 2.26 ms; n = 2900, m =
-// 2800, d = 16: 1.37 against 1.48), or, for one problem at d <= 10, also
-// streamed (n = m = 16000, d = 10: 11.9 against 16.8 ms; d = 16: 20.5 against
-// 16.8). A batch goes there when each of its
-// problems fits a cluster of 8 (96 problems up to 4096 points, d = 8, of
-// which a part had to go through the grid one by one: 12.8 against 7.6).
-bool rows_wanted(const ottb_problem* probs, int num, int d) {
-  const int D = rows_kernel(d).D;
-  if (D == 0) return false;
-  if (D <= 4 || (num == 1 && D <= 10)) return true;
-  auto fits = [](size_t bytes) { return bytes <= (size_t)kRowsSmemMax; };
-  if (num == 1)
-    return fits(rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true)) ||
-           fits(rows_smem(probs[0].n, probs[0].m, D, 148, kRowsWarps, false, true, true));
-  for (int i = 0; i < num; ++i)
-    if (!fits(rows_smem(probs[i].n, probs[i].m, D, 8, kRowsWarps, true, false))) return false;
-  return true;
-}
-
 // Clusters of `size` CTAs that the device holds at once. Cached: the query
 // stays out of later calls, which may be under stream capture.
 int rows_max_clusters(const void* fn, int size, int threads, size_t smem) {
@@ -521,7 +481,7 @@ int make_plan(const ottb_problem* probs, int num, int d, const ottb_solver_cfg* 
     plan.kern = pick_tc(plan.dp, 256);
   } else {
     plan.dp = simt_dp(d);
-    rows = rows_wanted(probs, num, d);
+    rows = rows_wanted(probs, num, rows_kernel(d).D, plan.dp);
     if (rows)
       plan.kern.fn = const_cast<void*>(rows_kernel(d).grid);
     else

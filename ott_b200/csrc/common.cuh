@@ -150,6 +150,28 @@ constexpr float kExp2C1 = 6.931469440e-01f;
 constexpr float kExp2C0 = 1.000000119e+00f;
 constexpr float kRoundShift = 12582912.0f;  // 1.5 * 2^23
 
+// 2^x on the FMA pipe, to take part of the exponentials off the MUFU pipe.
+// Range reduction x = n + f, n = rint(x), f in [-1/2, 1/2] (exact for
+// |x| < 2^22: adding 1.5 * 2^23 rounds x to an integer in the low mantissa
+// bits); 2^f by a degree-5 polynomial minimising the maximum relative error
+// on [-1/2, 1/2], fitted by tests/exp2_poly_fit.py (Remez exchange; 7.5e-8
+// minimax, 2.3e-7 evaluated in FP32); 2^n by adding n to the exponent
+// field. Inputs below -126 are clamped (the result, < 2^-125, is negligible
+// next to the running sum's leading term >= 1); callers keep x <= kTau + 1.
+__device__ __forceinline__ float exp2_poly(float x) {
+  x = fmaxf(x, -126.0f);
+  const float t = x + kRoundShift;
+  const float f = x - (t - kRoundShift);
+  float p = kExp2C5;
+  p = fmaf(p, f, kExp2C4);
+  p = fmaf(p, f, kExp2C3);
+  p = fmaf(p, f, kExp2C2);
+  p = fmaf(p, f, kExp2C1);
+  p = fmaf(p, f, kExp2C0);
+  // t's bits are 0x4B400000 + n; shifted left by 23 they are n << 23.
+  return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
+}
+
 // Packed pairs of FP32 values (sm_100 fma/add .f32x2: two lanes of FP32
 // arithmetic per instruction, same IEEE rounding as the scalar forms).
 typedef unsigned long long f32x2;
@@ -183,15 +205,8 @@ __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
   return r;
 }
 
-// 2^x for a pair on the FMA pipe, to take part of the exponentials off the
-// MUFU pipe.
-// Range reduction x = n + f, n = rint(x), f in [-1/2, 1/2] (exact for
-// |x| < 2^22: adding 1.5 * 2^23 rounds x to an integer in the low mantissa
-// bits); 2^f by a degree-5 polynomial minimising the maximum relative error
-// on [-1/2, 1/2], fitted by tests/exp2_poly_fit.py (Remez exchange; 7.5e-8
-// minimax, 2.3e-7 evaluated in FP32); 2^n by adding n to the exponent
-// field. Inputs below -126 are clamped (the result, < 2^-125, is negligible
-// next to the running sum's leading term >= 1); callers keep x <= kTau + 1.
+// exp2_poly on a pair, the range reduction and the polynomial in packed
+// arithmetic (same operations, same results as two exp2_poly calls).
 __device__ __forceinline__ f32x2 exp2_poly2(f32x2 xp) {
   float x0, x1;
   unpack2(xp, x0, x1);
@@ -242,11 +257,16 @@ __device__ __forceinline__ f32x2 exp2_poly2_d4(f32x2 xp) {
                __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23)));
 }
 
-// Of every 8 exponentials of the tensor-core epilogue's running-maximum path,
-// which runs its arithmetic on packed pairs, this many go to exp2_poly2
-// (measured in isolation, 16 warps per SM: 15.4 entries/clk/SM with scalar
-// FP32 and every exponential on the MUFU, 18.9 packed with 2 of 8 on the
-// polynomial, 15.6 with 4 of 8).
+// Of every 8 exponentials, this many go to exp2_poly: in the tiled CUDA-core
+// engine at d <= 4, where the MUFU pipe binds (measured at n = m = 32768,
+// d = 2: 2 of 8 is 2 % faster than 0, 3 of 8 slower; 8 problems of 100000 x
+// 8, d = 4: 10 %); and in the tensor-core epilogue's running-maximum path,
+// which runs its arithmetic on packed pairs (measured in isolation, 16 warps
+// per SM: 15.4 entries/clk/SM with scalar FP32 and every exponential on the
+// MUFU, 18.9 packed with 2 of 8 on the polynomial, 15.6 with 4 of 8).
+#ifndef OTTB_POLY_OF_8
+#define OTTB_POLY_OF_8 2
+#endif
 #ifndef OTTB_POLY_OF_8_TC
 #define OTTB_POLY_OF_8_TC 2
 #endif
@@ -254,9 +274,6 @@ __device__ __forceinline__ f32x2 exp2_poly2_d4(f32x2 xp) {
 // exp2_poly2 (a pair there costs the FMA pipe 16 cycles and takes 16 off the
 // MUFU, which binds only where the inner product is short).
 __host__ __device__ constexpr int rows_poly_pairs(int D) { return D <= 2 ? 2 : D == 3 ? 1 : 0; }
-#ifndef OTTB_POLY_OF_8_TC
-#define OTTB_POLY_OF_8_TC 2
-#endif
 
 // Order-preserving map of non-NaN floats to ints (and back), for atomic
 // maxima and minima of floats of either sign.

@@ -1,6 +1,6 @@
 // FP32 CUDA-core sweep engine, tiled: the calls that rows_wanted leaves it
-// (capi.cu; engine_rows.cuh serves the others). One work unit = 128 rows of A against a contiguous range of 128-column
-// tiles of B.
+// (fp32_route.h; engine_rows.cuh serves the others). One work unit = 128
+// rows of A against a contiguous range of 128-column tiles of B.
 //
 // The n x m cost never leaves registers. Each of the 256 threads owns an
 // 8 x 8 micro-tile (rows ty*4+{0..3}, 64+ty*4+{0..3}; columns tx*4+{0..3},
@@ -56,7 +56,6 @@ __device__ void simt_unit(SimtSmem<DP>& sm, const SweepOperands& op,
   const int tid = threadIdx.x;
   const int tx = tid & 15;
   const int ty = tid >> 4;
-
   // dot-product unrolling (registers are capped at 128 by two CTAs per SM)
   constexpr int kDotUnroll = DP <= 8 ? 2 : 4;
 
@@ -146,7 +145,11 @@ __device__ void simt_unit(SimtSmem<DP>& sm, const SweepOperands& op,
       }
       float e[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) e[j] = ex2_approx(acc[i][j] - mrow[i]);
+      for (int j = 0; j < 8; ++j) {
+        const float xj = acc[i][j] - mrow[i];
+        // small d is MUFU-bound: part of the exponentials on the FMA pipe
+        e[j] = (DP <= 4 && j >= 8 - OTTB_POLY_OF_8) ? exp2_poly(xj) : ex2_approx(xj);
+      }
       const float sum = ((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7]));
       two_sum_acc(lrow[i], lcmp[i], sum);
     }

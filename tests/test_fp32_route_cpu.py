@@ -1,0 +1,69 @@
+"""Which engine an FP32 call takes, against sizes at which one of the two
+measured clearly faster (B200; microseconds an iteration, tiled and
+row-owner)."""
+import os
+import subprocess
+
+import pytest
+
+from ott_b200 import build
+
+# n, m, number of problems, d, microseconds by the tiled and the row-owner engine
+_MEASURED = [
+    (200, 100000, 1, 2, 102, 182), (200, 100000, 1, 8, 138, 235), (100000, 200, 1, 4, 116, 205),
+    (1200, 100000, 1, 8, 261, 360), (2400, 100000, 1, 8, 420, 546), (600, 100000, 1, 8, 211, 271),
+    (300, 1000000, 1, 2, 1123, 1573), (150, 200000, 1, 3, 255, 363), (150, 200000, 1, 10, 389, 519),
+    (130, 40000, 1, 4, 76, 90), (400, 200000, 1, 10, 485, 527), (1800, 1000000, 1, 8, 3120, 3702), (900, 200000, 1, 8, 447, 551),
+    (20000, 30, 16, 2, 168, 679), (20000, 300, 16, 4, 261, 741), (20000, 1000, 16, 2, 398, 713),
+    (100000, 8, 8, 2, 559, 1343), (100000, 500, 4, 2, 583, 672), (6000, 6000, 32, 2, 1106, 1305),
+    (8, 4000, 1, 2, 64, 17), (4000, 200, 1, 2, 33, 20), (64, 100000, 1, 2, 1069, 177),
+    (10, 100000, 1, 8, 1678, 226), (8, 1000000, 1, 4, 12891, 1853), (16000, 16000, 1, 4, 332, 250),
+    (16000, 16000, 1, 8, 409, 357), (30000, 30000, 1, 10, 1839, 1178), (65536, 65536, 1, 8, 5902, 5250),
+    (131072, 131072, 1, 10, 33565, 21469), (2000, 40000, 1, 3, 235, 117), (700, 10000, 1, 8, 48, 43),
+    (9000, 40000, 1, 10, 873, 514), (12000, 200000, 1, 8, 3433, 2950), (20, 20000, 1, 2, 232, 47),
+    (2048, 2048, 1, 2, 24, 14), (7013, 5001, 1, 3, 120, 60), (120, 96, 1, 3, 15, 7),
+    (4000, 100, 64, 2, 135, 78), (8000, 8000, 4, 2, 301, 240), (60000, 1000, 2, 2, 341, 242),
+    (300000, 300, 2, 4, 1575, 1094), (1024, 1024, 256, 2, 500, 320), (5000, 700, 64, 4, 383, 308),
+]
+
+_MAIN = r"""
+#include <cstdio>
+#include <vector>
+#include "fp32_route.h"
+using namespace ottb;
+int main() {
+  for (const auto& c : kMeasured) {
+    std::vector<ottb_problem> p((size_t)c[2]);
+    for (auto& q : p) q.n = c[0], q.m = c[1];
+    const int d = (int)c[3];
+    const int dims[] = {2, 3, 4, 5, 6, 8, 10, 12, 16};
+    int D = 0, dp = 2;
+    for (int k : dims)
+      if (D == 0 && d <= k) D = k;
+    while (dp < d) dp <<= 1;
+    if (rows_wanted(p.data(), (int)p.size(), D, dp) != (c[5] < c[4]))
+      printf("%lld x %lld, %lld problems, d %d\n", c[0], c[1], c[2], d);
+  }
+  // beyond 32-bit row numbers
+  for (int64_t n : {((int64_t)1 << 30) + 1, (int64_t)1 << 31}) {
+    ottb_problem q{};
+    q.n = n, q.m = 10;
+    if (rows_wanted(&q, 1, 2, 2)) printf("n %lld\n", (long long)n);
+  }
+}
+"""
+
+
+def test_route_takes_the_faster_engine(tmp_path):
+  try:
+    nvcc = build.nvcc()
+  except RuntimeError:
+    pytest.skip("no nvcc")
+  rows = ",".join("{%s}" % ",".join(map(str, c)) for c in _MEASURED)
+  src, exe = tmp_path / "route.cu", tmp_path / "route"
+  src.write_text("static const long long kMeasured[][6] = {%s};\n%s" % (rows, _MAIN))
+  subprocess.run([nvcc, *build.ARCH, "-std=c++17", "-I", build.CSRC, "-o", str(exe), str(src)],
+                 check=True, capture_output=True, text=True)
+  run = subprocess.run([str(exe)], capture_output=True, text=True, check=True,
+                       env={**os.environ, "CUDA_VISIBLE_DEVICES": ""})
+  assert run.stdout == "", run.stdout

@@ -268,3 +268,25 @@ def test_large_streamed_dimensions(n, m, d):
   np.testing.assert_allclose(out.f.cpu().numpy(), f.cpu().numpy(), rtol=0, atol=1e-4 * eps)
   np.testing.assert_allclose(out.g.cpu().numpy(), g.cpu().numpy(), rtol=0, atol=1e-4 * eps)
   np.testing.assert_allclose(float(out.errors[0]), err, rtol=1e-2, atol=1e-6)
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 4])
+@pytest.mark.parametrize("n,m", [(150, 40001), (60003, 200)])
+def test_short_sides_of_long_problems(n, m, d):
+  """Left to the tiled engine, at its smallest dimensions."""
+  _check(n, m, d, seed=d, max_iterations=20)
+
+
+def test_batch_of_long_problems():
+  """Several problems that would take the whole grid one after another: the
+  tiled engine, with small ones between."""
+  import torch
+  from ott_b200.geometry import pointcloud
+  from ott_b200.solvers import linear
+  ps = [problems.uniform_cloud_problem(n, m, 3, seed=n)
+        for n, m in [(20000, 30), (20003, 301), (45, 21000), (300, 200)]]
+  cu = lambda t: torch.as_tensor(t).cuda()  # noqa: E731
+  geoms = [pointcloud.PointCloud(cu(p[0]), cu(p[1]), epsilon=0.05) for p in ps]
+  outs = linear.solve_batch(geoms, [cu(p[2]) for p in ps], [cu(p[3]) for p in ps])
+  for p, geom, out in zip(ps, geoms, outs):
+    helpers.assert_parity(geom, out, helpers.oracle_solve(*p, epsilon=0.05, batch_size=1024))

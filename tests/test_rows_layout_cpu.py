@@ -41,7 +41,7 @@ int main() {
 def test_streamed_layout_fits(tmp_path):
   try:
     nvcc = build.nvcc()
-  except Exception:  # noqa: BLE001
+  except RuntimeError:
     pytest.skip("no nvcc")
   src, exe = tmp_path / "layout.cu", tmp_path / "layout"
   src.write_text(_SRC)
