@@ -395,6 +395,14 @@ class _Potentials(torch.autograd.Function):
             cast(gb, p.b, 3), None, None, None, None, None)
 
 
+def _has_storage(t: torch.Tensor) -> bool:
+  try:
+    t.data_ptr()
+  except RuntimeError:
+    return False
+  return True
+
+
 class _RegOTCost(torch.autograd.Function):
   """``reg_ot_cost`` of a solved problem as a function of ``(x, y, a, b)``,
   its backward the gradient with the potentials held fixed
@@ -409,8 +417,10 @@ class _RegOTCost(torch.autograd.Function):
   @torch.autograd.function.once_differentiable
   def backward(ctx, gout):  # pylint: disable=arguments-differ
     need = ctx.needs_input_grad
-    if ctx.out.geom._scale_cost != "mean":
+    if ctx.out.geom._scale_cost != "mean" and _has_storage(gout):
       return (*ctx.out._fixed_potential_grads(need[:4], gout, torch.float32), None)
+    # a batched gout (is_grads_batched, a vectorized jacobian) has no memory
+    # for a kernel to read: the gradients once, scaled by tensor operations
     gx, gy, ga, gb = ctx.out.reg_ot_cost_grads()
     cast = lambda t, i: (gout * t).to(torch.float32) if need[i] else None
     return cast(gx, 0), cast(gy, 1), cast(ga, 2), cast(gb, 3), None

@@ -37,3 +37,29 @@ def test_matches_tensor_formula(n, m, d):
       assert g.dtype == torch.float32
       ref = -0.75 * w
       assert float((g.double() - ref).abs().max()) <= 2.0 ** -23 * max(float(ref.abs().max()), 1e-30)
+
+
+def test_batched_grad_outputs():
+  """is_grads_batched and a vectorized jacobian: the scaled gradients, each
+  with one float32 rounding, as one call after another."""
+  import torch
+  from ott_b200.geometry import pointcloud
+  from ott_b200.solvers import linear
+  x, y, a, b = (torch.as_tensor(t).cuda() for t in problems.uniform_cloud_problem(40, 50, 3, seed=1))
+  x.requires_grad_()
+  a.requires_grad_()
+  cost = lambda x: linear.reg_ot_cost(pointcloud.PointCloud(x, y, epsilon=0.1), a, b)  # noqa: E731
+  c = cost(x)
+  scales = torch.tensor([1.0, -2.0, 3.0], dtype=torch.float64, device="cuda")
+  batched = torch.autograd.grad(c, [x, a], grad_outputs=scales, is_grads_batched=True,
+                                retain_graph=True)
+  for k, s in enumerate(scales):
+    one = torch.autograd.grad(c, [x, a], grad_outputs=s, retain_graph=True)
+    for got, want in zip(batched, one):
+      bound = 2.0 ** -23 * float(want.abs().max())
+      assert float((got[k] - want).abs().max()) <= bound
+  two = lambda x: torch.stack([cost(x), 2 * cost(x)])  # noqa: E731
+  jac = torch.autograd.functional.jacobian
+  want = jac(two, x)
+  assert float((jac(two, x, vectorize=True) - want).abs().max()) <= \
+      2.0 ** -23 * float(want.abs().max())
