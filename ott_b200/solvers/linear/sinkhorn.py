@@ -280,6 +280,10 @@ class SinkhornOutput(NamedTuple):
     x, y = geom.x.detach(), geom.y.detach()
     dev = x.device
     a, b, f, g = (_arrays.as_f32(t, dev).detach() for t in (self.a, self.b, self.f, self.g))
+    # the kernels below know the lengths only
+    for name, t, cnt in (("a", a, n), ("b", b, m), ("f", f, n), ("g", g, m)):
+      if t.numel() != cnt:
+        raise ValueError(f"{name} must have length {cnt}, got shape {tuple(t.shape)}")
     new = lambda flag, like: torch.empty_like(like, dtype=dtype) if flag else None  # noqa: E731
     gx, gy, ga, gb = new(need[0], x), new(need[1], y), new(need[2], a), new(need[3], b)
 

@@ -63,3 +63,14 @@ def test_batched_grad_outputs():
   want = jac(two, x)
   assert float((jac(two, x, vectorize=True) - want).abs().max()) <= \
       2.0 ** -23 * float(want.abs().max())
+
+
+def test_potentials_of_another_length():
+  """Refused, as the tensor formula's arithmetic refuses them, before a
+  kernel reads them."""
+  import torch
+  x, y, a, b = problems.uniform_cloud_problem(40, 50, 3, seed=1)
+  _, out = helpers.gpu_solve(x, y, a, b, epsilon=0.3)
+  for wrong in ((out.f[:-1], out.g), (out.f, torch.cat([out.g, out.g]))):
+    with pytest.raises(ValueError):
+      out._replace(potentials=wrong).reg_ot_cost_grads()
