@@ -400,7 +400,8 @@ __device__ __forceinline__ bool grid_barrier(Globals* gl, unsigned expected,
   if (threadIdx.x == 0) {
     const unsigned long long target = ++bar.phase * expected;
     // release and acquire at gpu scope are cumulative over the CTA's
-    // __syncthreads: no separate fences
+    // __syncthreads: no separate fences. They cover generic accesses only;
+    // what TMA loads read behind the barrier has tc::fence_proxy_async_global.
     unsigned long long* ctr = &gl->bar_count;
     asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(ctr) : "memory");
     auto poll = [&]() {

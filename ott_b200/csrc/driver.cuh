@@ -13,6 +13,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tc_ptx.cuh"
 
 namespace ottb {
 
@@ -323,6 +324,7 @@ __device__ __forceinline__ void finalize_rows_warp(const ProbDev& P, const Sweep
         }
       }
     }
+    if (ext) tc::fence_proxy_async_global();  // the next sweep's TMA loads read the shifts
     if (P.dkey && !P.symmetric) {
       for (int off = 16; off > 0; off >>= 1) {
         dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, off));

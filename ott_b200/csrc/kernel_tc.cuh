@@ -333,6 +333,9 @@ __device__ bool tc_sweep(const KernelArgs& A, const SweepParams& sp, unsigned sw
     }
   } else if (warp < 2) {
     // producer (warp 0) and MMA issuer (warp 1)
+    // the column shifts, which other CTAs wrote with plain stores in the last
+    // sweep, before this one's TMA loads of them
+    if (warp == 0) tc::fence_proxy_async_global();
     while (true) {
       const uint32_t d = pp.desc++;
       const uint32_t slot = d % NSLOT;

@@ -232,6 +232,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Orders generic-proxy accesses to global memory before this fence against
+// async-proxy accesses (TMA loads) after it, in either direction. A release
+// and an acquire order generic accesses only: values written with plain
+// stores and read by TMA elsewhere take this fence behind the stores and
+// ahead of the loads.
+__device__ __forceinline__ void fence_proxy_async_global() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
+
 // Instruction descriptor, kind::f16: D f32 (bits 4-5 = 1), A and B bf16
 // (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in
 // bits 17-22, M >> 4 in bits 24-28.
