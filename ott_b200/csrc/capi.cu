@@ -362,16 +362,11 @@ int rows_max_clusters(const void* fn, int size, int threads, size_t smem) {
   return n;
 }
 
-// Team sizes of the row-owner engine, from a model of one sweep in SM
-// cycles: entries x cycles per entry / CTAs, plus what a sweep costs beyond
-// its entries (column shifts, lane and warp merges, the update in FP64, the
-// team's barrier).
+// Team sizes of the row-owner engine (rows_teams) and the mode of its grid.
 int plan_rows(Plan& plan, int d, const DeviceInfo& di) {
   RowsPlan& R = plan.rows;
   R.kern = rows_kernel(d);
   const int D = R.kern.D;
-  const double per_entry = D <= 4 ? 0.105 : (D + 8) / 75.0;
-  const double over_one = 4500, over_cluster = 5500, over_grid = 11000, over_warp = 100;
   const int num = plan.num;
   if (!ensure_dynamic_smem(R.kern.grid, kRowsSmemMax) ||
       !ensure_dynamic_smem(R.kern.cluster, kRowsSmemMax))
@@ -383,56 +378,19 @@ int plan_rows(Plan& plan, int d, const DeviceInfo& di) {
     const int64_t slots = (int64_t)std::min<size_t>(pp.off_arr - pp.off_pm, kRowsKeyBytes) / 16;
     return (int)std::max<int64_t>(1, std::min(g, std::max<int64_t>(pp.rb_g, slots)));
   };
-  auto entries = [&](const ProbPlan& pp) { return (double)pp.n * (double)pp.m * per_entry; };
-  // cost[k]: the k largest problems by the whole grid, the rest by clusters
-  std::vector<double> grid_t(num + 1, 0.0);
-  for (int t = 0; t < num; ++t)
-    grid_t[t + 1] = grid_t[t] + entries(plan.probs[t]) / grid_size(plan.probs[t]) + over_grid;
-  double best = grid_t[num];
-  int best_k = num;
-  for (int C = 1; C <= kRowsMaxCluster; C *= 2) {
-    for (int threads = kRowsThreads; threads >= 128; threads /= 2) {
-      const int warps = threads / 32;
-      double sum = 0.0, longest = 0.0;
-      size_t smem = 0;
-      for (int k = num - 1; k >= 0; --k) {
-        const ProbPlan& pp = plan.probs[k];
-        smem = std::max(smem, rows_smem(pp.n, pp.m, D, C, warps, true, false));
-        if (smem > kRowsSmemMax) break;
-        // CTAs that share an SM share its pipes; one alone needs about ten
-        // warps to fill them
-        const int per_sm = std::min<int>(kRowsThreads / threads,
-                                         (int)(kRowsSmemMax / (smem + rows_static_smem() + 1024)));
-        // large clusters leave SMs of a GPC over (7 of 9 clusters of 16 fit)
-        const double slots = (double)di.sms * std::max(per_sm, 1) / C *
-                             (C >= 8 ? 0.78 : C >= 4 ? 0.88 : 1.0);
-        const double alone = std::min(1.0, warps / 10.0);
-        const double share = std::max(1.0, std::min((double)per_sm, (num - k) * C / (double)di.sms));
-        const double t = entries(pp) / C / std::min(alone, 1.0 / share) +
-                         (C > 1 ? over_cluster : over_one) + over_warp * warps;
-        sum += t;
-        longest = std::max(longest, t);
-        // problems stop at different iterations: a batch ends with its
-        // longest-running ones
-        const double est = num - k == 1 ? t : std::max(longest, sum / slots + longest);
-        if (grid_t[k] + est < best) {
-          best = grid_t[k] + est;
-          best_k = k;
-          R.csize = C;
-          R.cthreads = threads;
-          R.csmem = smem;
-        }
-      }
-    }
-  }
+  std::vector<RowsSize> sizes;
+  for (const ProbPlan& pp : plan.probs) sizes.push_back(RowsSize{pp.n, pp.m, grid_size(pp)});
+  const RowsTeams teams = rows_teams(
+      sizes, D, di.sms, rows_static_smem(), [&](int size, int threads, size_t smem) {
+        return rows_max_clusters(R.kern.cluster, size, threads, smem);
+      });
+  R.csize = teams.csize;
+  R.cthreads = teams.cthreads;
+  R.csmem = teams.csmem;
+  R.nclusters = teams.nclusters;
   R.grid.clear();
   R.cluster.clear();
-  for (int t = 0; t < num; ++t) (t < best_k ? R.grid : R.cluster).push_back(t);
-  if (!R.cluster.empty()) {
-    R.nclusters = rows_max_clusters(R.kern.cluster, R.csize, R.cthreads, R.csmem);
-    if (R.nclusters < 1) return OTTB_ERR_CUDA;
-    R.nclusters = std::min<int>(R.nclusters, (int)R.cluster.size());
-  }
+  for (int t = 0; t < num; ++t) (t < teams.grid ? R.grid : R.cluster).push_back(t);
   if (!R.grid.empty()) {
     R.gsize = di.sms;
     for (int t : R.grid) R.gsize = std::min(R.gsize, grid_size(plan.probs[t]));

@@ -1,10 +1,11 @@
-// Which engine an FP32 call takes: the row-owner engine (engine_rows.cuh) or
-// the tiled one (engine_simt.cuh), from the sizes alone.
+// Which engine an FP32 call takes, from the sizes alone: the row-owner engine
+// (engine_rows.cuh), and with which teams, or the tiled one (engine_simt.cuh).
 #pragma once
 
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <vector>
 
 #include "rows.h"
 
@@ -133,6 +134,82 @@ inline bool rows_wanted(const ottb_problem* probs, int num, int D, int dp) {
       grid += rows_grid_us(n, m, D);
   }
   return grid == 0.0 || grid <= tiled_us(probs, num, dp);
+}
+
+// Problem of a call, and the CTAs that the whole grid would solve it with.
+struct RowsSize {
+  int64_t n, m;
+  int grid_ctas;
+};
+
+// Teams of a call: the first `grid` problems one after another by the whole
+// grid, the others drawn by clusters of `csize` CTAs.
+struct RowsTeams {
+  int grid = 0, csize = 1, cthreads = 0, nclusters = 0;
+  size_t csmem = 0;
+};
+
+// Team sizes of the row-owner engine for problems in decreasing work, from a
+// model of one sweep in SM cycles: entries x cycles per entry / CTAs, plus
+// what a sweep costs beyond its entries (column shifts, lane and warp merges,
+// the update in FP64, the team's barrier). clusters(size, threads, smem): how
+// many clusters the device holds at once; where it holds none of the best
+// size (SMs of a GPC left to others), smaller ones and the grid are tried.
+template <class Clusters>
+inline RowsTeams rows_teams(const std::vector<RowsSize>& probs, int D, int sms, size_t static_smem,
+                            Clusters clusters) {
+  const double per_entry = D <= 4 ? 0.105 : (D + 8) / 75.0;
+  const double over_one = 4500, over_cluster = 5500, over_grid = 11000, over_warp = 100;
+  const int num = (int)probs.size();
+  auto entries = [&](const RowsSize& p) { return (double)p.n * (double)p.m * per_entry; };
+  // grid_t[k]: the k largest problems by the whole grid
+  std::vector<double> grid_t(num + 1, 0.0);
+  for (int t = 0; t < num; ++t)
+    grid_t[t + 1] = grid_t[t] + entries(probs[t]) / probs[t].grid_ctas + over_grid;
+  for (int most = kRowsMaxCluster;;) {
+    RowsTeams T;
+    T.grid = num;
+    double best = grid_t[num];
+    for (int C = 1; C <= most; C *= 2) {
+      for (int threads = kRowsThreads; threads >= 128; threads /= 2) {
+        const int warps = threads / 32;
+        double sum = 0.0, longest = 0.0;
+        size_t smem = 0;
+        for (int k = num - 1; k >= 0; --k) {
+          const RowsSize& p = probs[k];
+          smem = std::max(smem, rows_smem(p.n, p.m, D, C, warps, true, false));
+          if (!rows_fits(smem)) break;
+          // CTAs that share an SM share its pipes; one alone needs about ten
+          // warps to fill them
+          const int per_sm = std::min<int>(kRowsThreads / threads,
+                                           (int)(kRowsSmemMax / (smem + static_smem + 1024)));
+          // large clusters leave SMs of a GPC over (7 of 9 clusters of 16 fit)
+          const double slots = (double)sms * std::max(per_sm, 1) / C *
+                               (C >= 8 ? 0.78 : C >= 4 ? 0.88 : 1.0);
+          const double alone = std::min(1.0, warps / 10.0);
+          const double share = std::max(1.0, std::min((double)per_sm, (num - k) * C / (double)sms));
+          const double t = entries(p) / C / std::min(alone, 1.0 / share) +
+                           (C > 1 ? over_cluster : over_one) + over_warp * warps;
+          sum += t;
+          longest = std::max(longest, t);
+          // problems stop at different iterations: a batch ends with its
+          // longest-running ones
+          const double est = num - k == 1 ? t : std::max(longest, sum / slots + longest);
+          if (grid_t[k] + est < best) {
+            best = grid_t[k] + est;
+            T.grid = k;
+            T.csize = C;
+            T.cthreads = threads;
+            T.csmem = smem;
+          }
+        }
+      }
+    }
+    if (T.grid == num) return T;
+    T.nclusters = std::min(clusters(T.csize, T.cthreads, T.csmem), num - T.grid);
+    if (T.nclusters > 0) return T;
+    most = T.csize / 2;
+  }
 }
 
 }  // namespace ottb

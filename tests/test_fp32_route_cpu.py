@@ -54,16 +54,48 @@ int main() {
 """
 
 
-def test_route_takes_the_faster_engine(tmp_path):
+_TEAMS = r"""
+#include <cstdio>
+#include <vector>
+#include "fp32_route.h"
+using namespace ottb;
+int main() {
+  // a device that holds clusters of at most `fit` CTAs at once, or none
+  for (int fit : {16, 8, 4, 2, 1, 0}) {
+    auto clusters = [&](int size, int, size_t) { return size <= fit ? 9 : 0; };
+    for (int num : {1, 3, 40}) {
+      std::vector<RowsSize> p;
+      for (int i = 0; i < num; ++i) p.push_back(RowsSize{1500 - 10 * i, 900, 148});
+      const RowsTeams T = rows_teams(p, 3, 148, 2500, clusters);
+      const bool on_grid = T.grid == num;
+      if (on_grid ? T.nclusters != 0 : T.csize > fit || T.nclusters < 1 || !rows_fits(T.csmem))
+        printf("fit %d, %d problems: grid %d, %d clusters of %d\n", fit, num, T.grid, T.nclusters,
+               T.csize);
+    }
+  }
+}
+"""
+
+
+def _run(tmp_path, source):
   try:
     nvcc = build.nvcc()
   except RuntimeError:
     pytest.skip("no nvcc")
-  rows = ",".join("{%s}" % ",".join(map(str, c)) for c in _MEASURED)
   src, exe = tmp_path / "route.cu", tmp_path / "route"
-  src.write_text("static const long long kMeasured[][6] = {%s};\n%s" % (rows, _MAIN))
+  src.write_text(source)
   subprocess.run([nvcc, *build.ARCH, "-std=c++17", "-I", build.CSRC, "-o", str(exe), str(src)],
                  check=True, capture_output=True, text=True)
-  run = subprocess.run([str(exe)], capture_output=True, text=True, check=True,
+  run = subprocess.run([str(exe)], capture_output=True, text=True, check=True, timeout=120,
                        env={**os.environ, "CUDA_VISIBLE_DEVICES": ""})
   assert run.stdout == "", run.stdout
+
+
+def test_a_device_without_room_for_the_best_cluster(tmp_path):
+  """Smaller clusters, or the grid: no call is refused for it."""
+  _run(tmp_path, _TEAMS)
+
+
+def test_route_takes_the_faster_engine(tmp_path):
+  rows = ",".join("{%s}" % ",".join(map(str, c)) for c in _MEASURED)
+  _run(tmp_path, "static const long long kMeasured[][6] = {%s};\n%s" % (rows, _MAIN))
