@@ -158,7 +158,9 @@ int32_t ottb_sinkhorn_launch(const ottb_problem* problems, int32_t num_problems,
  * solve twice (one untimed, one timed with CUDA events), writing the
  * problems' outputs and results; the call blocks until the trials finish
  * and refuses a stream under capture (OTTB_ERR_INVALID). Returns at once if
- * the shape is already tuned, unless force != 0. */
+ * the shape is already tuned, unless force != 0. FP32 calls on the row-owner
+ * engine (most of d <= 10, and larger d where the points stay in shared
+ * memory) have no schedule to choose: one solve, nothing to tune. */
 int32_t ottb_sinkhorn_autotune(const ottb_problem* problems, int32_t num_problems,
                                int32_t d, const ottb_solver_cfg* cfg,
                                ottb_result* results, void* workspace,
@@ -176,7 +178,9 @@ int32_t ottb_sinkhorn_autotune(const ottb_problem* problems, int32_t num_problem
  * dynamic: 1 deals work units from an
  * atomic queue, 0 round-robin (calls with several problems always queue);
  * tile_n: columns of a tensor-core tile, 256 or 128 (ignored by the
- * CUDA-core engine). OTTB_ERR_INVALID for values outside those ranges. */
+ * CUDA-core engine). Calls on the row-owner engine
+ * (ottb_sinkhorn_autotune) take no schedule: the record has no effect there.
+ * OTTB_ERR_INVALID for values outside those ranges. */
 int32_t ottb_sinkhorn_set_schedule(const ottb_problem* problems, int32_t num_problems,
                                    int32_t d, const ottb_solver_cfg* cfg,
                                    int32_t split_scale, int32_t waves, int32_t dynamic,

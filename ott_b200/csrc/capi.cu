@@ -1094,10 +1094,12 @@ int32_t ottb_sinkhorn_autotune(const ottb_problem* problems, int32_t num_problem
   // round-robin or queued units; the split stays as chosen); for several
   // problems, how far the splits of the problems still
   // iterating may grow (0, 1, 2, 4 waves of units). On the tensor cores each
-  // of these with 256- and with 128-column tiles.
+  // of these with 256- and with 128-column tiles. The row-owner engine has
+  // no such choice: the one solve, for the outputs.
   std::vector<Schedule> cands;
+  if (base.rows.on) cands.push_back(base.sched);
   for (int tile : {256, 128}) {
-    if (tile != 256 && !base.tc) break;
+    if (base.rows.on || (tile != 256 && !base.tc)) break;
     if (num_problems == 1) {
       for (int scale : {4, 2, 8})
         for (int dyn : {0, 1}) {
@@ -1132,7 +1134,7 @@ int32_t ottb_sinkhorn_autotune(const ottb_problem* problems, int32_t num_problem
     if (st != OTTB_OK) break;
     st = write_header(problems, num_problems, cfg, plan, (char*)workspace, stream);
     // one untimed run, then one timed run of the whole solve
-    for (int rep = 0; rep < 2 && st == OTTB_OK; ++rep) {
+    for (int rep = base.rows.on ? 1 : 0; rep < 2 && st == OTTB_OK; ++rep) {
       if (rep == 1 && cudaEventRecord(e0, stream) != cudaSuccess) st = OTTB_ERR_CUDA;
       if (st == OTTB_OK)
         st = launch_solve(num_problems, d, cfg, results, plan, (char*)workspace, stream);
