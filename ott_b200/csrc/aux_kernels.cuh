@@ -20,8 +20,11 @@ struct PrepArgs {
 };
 
 // Threads of the centre's CTA: with 1024, d = 64 takes one round of loads a
-// side (256 threads: four).
+// side (256 threads: four; 18.7 -> 8.6 us). At short dimensions 256 are one
+// round already, and more only lengthen the sum over them (d = 2: 9.5 us with
+// 1024, 6.0 with 256).
 constexpr int kCenterThreads = 1024;
+__host__ __device__ constexpr int center_threads(int d) { return d <= 16 ? 256 : kCenterThreads; }
 
 // Common centre of the two clouds: the midpoint of the means of strided
 // samples (at most 256 points each) of x and y. C_ij = |x_i - y_j|^2 does

@@ -768,7 +768,7 @@ int launch_solve(int num_problems, int d, const ottb_solver_cfg* cfg, ottb_resul
   {
     PrepArgs pa{d_ptrs, d_probs, d, plan.dp};
     // the common centre once per problem, then the points
-    center_kernel<<<num_problems, kCenterThreads, 0, stream>>>(pa);
+    center_kernel<<<num_problems, center_threads(d), 0, stream>>>(pa);
     int64_t mx = 1;
     for (const ProbPlan& pp : plan.probs) mx = std::max(mx, std::max(pp.n_pad, pp.m_pad));
     // one thread per row (FP32 layout) or one warp per row, 8 rows a warp
