@@ -242,9 +242,10 @@ bool wants_tc(const ottb_solver_cfg* cfg, int d) {
   return cfg->precision == OTTB_PRECISION_AUTO && d >= 32;
 }
 
-// How the row-owner engine runs an FP32 call (engine_rows.cuh, rows_wanted). The problems of `cluster` are drawn by thread-block
-// clusters of `csize` CTAs, those of `grid` are solved one after another by
-// the whole grid; both are table positions in decreasing work.
+// How the row-owner engine runs an FP32 call (engine_rows.cuh, rows_wanted).
+// The problems of `cluster` are drawn by thread-block clusters of `csize`
+// CTAs, those of `grid` are solved one after another by the whole grid; both
+// are table positions in decreasing work.
 struct RowsPlan {
   bool on = false;
   RowsKernel kern;

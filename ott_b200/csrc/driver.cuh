@@ -218,8 +218,9 @@ __device__ void finalize_rows_g(const ProbDev& P, const SweepParams& sp, int par
   }
 }
 
-// What the update of N rows a lane (lane l: rows row0 + l + 32 k) reads that does not depend on the sweep: loaded while the warp
-// waits for the sweep's sums.
+// What the update of N rows a lane (lane l: rows row0 + l + 32 k) reads that
+// does not depend on the sweep: loaded while the warp waits for the sweep's
+// sums.
 template <int N>
 struct RowInputs {
   float nrm[N], old[N];

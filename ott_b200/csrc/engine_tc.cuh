@@ -78,7 +78,10 @@ struct TcCfg {
   static constexpr int kThreads = 32 * (kCtrlWarps + kEpiWarps);
   static constexpr int kDescSlots = 4;    // unit descriptors in flight
   // problem records kept in shared memory (a record read through an L1 that
-  // every barrier's acquire empties costs the control warps trips to L2)
+  // every barrier's acquire empties costs the control warps trips to L2): what
+  // fits beside the other buffers, in round numbers. A call has all of its
+  // records there or none, so one of more problems reads every record from
+  // global memory.
   static constexpr int kProbSlots = DK == 64 ? 112 : 4;
   static constexpr uint32_t kIdesc = tc::idesc_bf16_f32(128, kTileN);
   // extension blocks: R rows x 16 bf16, K-major without swizzle: K half 0

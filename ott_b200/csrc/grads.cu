@@ -3,7 +3,7 @@
 // include/ott_b200.h).
 //
 // Bound by launches, not by bytes: the same arithmetic written with tensor
-// operations takes about sixty small kernels (0.5 ms of host time a term at
+// operations takes about fifty small kernels (0.5 ms of host time a term at
 // n = m = 4096, d = 64, where the bytes take 1 us); here it takes one launch
 // for the points and two for the weights.
 #include <cuda_runtime.h>

@@ -177,10 +177,11 @@ __host__ __device__ inline RowsLayout rows_layout(int64_t n, int64_t m, int D, i
 // reads none of its values: with n = 4000, m = 200 on 148 CTAs, 98 own no
 // row of y and publish nothing in g-sweeps, so nothing would hold back the
 // f-sweep that overwrites what they read. Every CTA with rows reads every
-// word: measured on B200, a sweep of n = m = 2048, d = 2 takes 12.1 k cycles
-// with words and 13.9 k with the barrier; of n = 7013, m = 5001, d = 3, 56 k
-// with words and 43 k with the barrier (148 CTAs poll 56 KB each). Hence the
-// limit on n + m.
+// word, so the words lose where there are many: an iteration of n = m, d = 2
+// takes, with words and with the barrier, 16.9 and 19.2 us at 1000, 18.3 and
+// 20.8 at 2000, 27.5 and 24.3 at 2500, 24.2 and 26.6 at 3000, 27.5 and 29.6
+// at 4000, 55 and 39 at 5000, 61 and 47 at 6000 (B200; d = 4 and 8 alike):
+// they turn between n + m = 8000 and 10000. The limit lies below that.
 constexpr int64_t kRowsWordsMax = 6000;
 constexpr size_t kRowsSumBytes = 4096;  // 2 doubles a CTA (up to kRowsMaxCtas), the keys
 __host__ __device__ __forceinline__ size_t rows_words_bytes(int64_t n, int64_t m) {
