@@ -432,6 +432,8 @@ struct RowsShared {
   int iters[2];          // ... and its iterations per warp
   int row0[2], row1[2];  // this CTA's rows, per sweep kind
   unsigned owners[2];    // cluster, per sweep kind: bit q, CTA q owns rows of it
+  unsigned awaits;       // cluster, bit k of bar[k]: this CTA is sent those values
+  int partial;           // a CTA of the team owns no rows of one sweep kind
   int resync;            // see sums
   double red[2][kRowsWarps];
   double slot[2][kRowsMaxCluster];  // cluster: each CTA's error and marginal sums
@@ -501,17 +503,25 @@ struct RowsSolver {
       rows_sh.iters[kind] = rows_iters(rows_sh.cover[kind], (G + W - 1) >> wsh, rows_groups(D));
     }
     if (threadIdx.x < 2) rows_sh.bound[threadIdx.x] = 0;
-    if (threadIdx.x < 32) {
-      const int q = threadIdx.x, size = rows_sh.size;
-      for (int kind = 0; kind < 2; ++kind) {
-        const int64_t rows = kind == kSweepG ? P.m : P.n;
-        const unsigned mask = __ballot_sync(
-            0xffffffffu, q < size && rows_begin(rows, q, size) < rows_begin(rows, q + 1, size));
-        if (q == 0) rows_sh.owners[kind] = mask;
-      }
-      if (q == 0)
-        rows_sh.resync = (min(P.n, P.m) + 3) / 4 < size ||
-                         (P.symmetric && rows_sh.A.cfg.inner_iterations == 1);
+    // A side with fewer quads of rows than the team has CTAs leaves some
+    // without rows.
+    const bool partial = (min(P.n, P.m) + 3) / 4 < rows_sh.size;
+    if (threadIdx.x == 0) {
+      rows_sh.partial = partial;
+      rows_sh.resync = partial || (P.symmetric && rows_sh.A.cfg.inner_iterations == 1);
+      // x's values are read by g-sweeps, y's by f-sweeps (in a symmetric
+      // problem, where every CTA owns the same rows of both, by g-sweeps)
+      rows_sh.awaits =
+          rows_sh.size == 1 ? 0u : (has_rows(kSweepG) ? 1u : 0u) | (has_rows(kSweepF) ? 6u : 0u);
+    }
+    // (by a loop: a ballot here, executed or not, cost the sweeps of 256
+    // problems of 1024 points 2 %)
+    if (!GRID && partial && threadIdx.x < 2) {
+      const int64_t rows = threadIdx.x == kSweepG ? P.m : P.n;
+      unsigned mask = 0;
+      for (int q = 0; q < rows_sh.size; ++q)
+        if (rows_begin(rows, q, rows_sh.size) < rows_begin(rows, q + 1, rows_sh.size)) mask |= 1u << q;
+      rows_sh.owners[threadIdx.x] = mask;
     }
     const int x0 = rows_sh.row0[kSweepF], x1 = rows_sh.row1[kSweepF];
     const int y0 = rows_sh.row0[kSweepG], y1 = rows_sh.row1[kSweepG];
@@ -719,9 +729,7 @@ struct RowsSolver {
     if (cmd.write) {
       const int to = isf ? 0 : 1 + (cmd.parity ^ 1);
       S.seq_of[to] = cmd.seq;
-      // x's values are read by g-sweeps, y's by f-sweeps (in a symmetric
-      // problem, where every CTA owns the same rows of both, by g-sweeps)
-      if (!GRID && rows_sh.size > 1 && has_rows(isf ? kSweepG : kSweepF)) S.pending |= 1u << to;
+      if (!GRID) S.pending |= 1u << to & rows_sh.awaits;
     }
     cmd.mult = mult;
     cmd.ws = mult == 1.0f ? P.ws_t : sweep_wscale(P, mult);
@@ -1035,9 +1043,15 @@ struct RowsSolver {
           if (lead) *dst = x;
         } else {
           const uint64_t* b = &rows_sh.bar[isG ? 1 + (parity ^ 1) : 0];
-          const unsigned readers = rows_sh.owners[isG ? kSweepF : kSweepG];
-          for (int q = k; q < rows_sh.size; q += lanes)
-            if (readers >> q & 1) cluster_store_async(cluster_addr(dst, q), x, cluster_addr(b, q));
+          // only to the CTAs that own rows of the sweep that reads them
+          if (!rows_sh.partial) {
+            for (int q = k; q < rows_sh.size; q += lanes)
+              cluster_store_async(cluster_addr(dst, q), x, cluster_addr(b, q));
+          } else {
+            const unsigned readers = rows_sh.owners[isG ? kSweepF : kSweepG];
+            for (int q = k; q < rows_sh.size; q += lanes)
+              if (readers >> q & 1) cluster_store_async(cluster_addr(dst, q), x, cluster_addr(b, q));
+          }
         }
       }
       if (lead && L.own) rows_mem[(isG ? L.py + (parity ^ 1) * L.rg : L.px) + own] = nf;
