@@ -48,7 +48,12 @@ inline bool rows_resident(int64_t n, int64_t m, int D) {
 // 131072 points a side.
 inline double rows_grid_us(int64_t n, int64_t m, int D) {
   const double entry =  // an entry of a CTA
-      1e-3 * (D <= 2 ? 0.044 : D == 3 ? 0.047 : D == 4 ? 0.050 : D <= 6 ? 0.065 : D <= 8 ? 0.075 : 0.090);
+      1e-3 * (D <= 2   ? 0.044
+              : D == 3 ? 0.047
+              : D == 4 ? 0.050
+              : D <= 6 ? 0.065
+              : D <= 8 ? 0.075
+                       : 0.090);
   const bool res = rows_resident(n, m, D);
   double t = 0.0;
   for (int side = 0; side < 2; ++side) {
@@ -66,7 +71,8 @@ inline double rows_grid_us(int64_t n, int64_t m, int D) {
 // without one and grow it to 8 (an average of about 4) while they offer less
 // than two units a CTA.
 inline double tiled_us(const ottb_problem* probs, int num, int dp) {
-  const double tile = dp <= 2 ? 1.95 : dp <= 4 ? 2.4 : dp <= 8 ? 3.1 : 4.6;  // by one CTA of two an SM
+  // a tile, by one CTA of two an SM
+  const double tile = dp <= 2 ? 1.95 : dp <= 4 ? 2.4 : dp <= 8 ? 3.1 : 4.6;
   const double unit = 7.5, sweep = 8.8;
   double t = 0.0;
   for (int side = 0; side < 2; ++side) {
