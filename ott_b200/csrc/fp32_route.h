@@ -165,8 +165,16 @@ template <class Clusters>
 inline RowsTeams rows_teams(const std::vector<RowsSize>& probs, int D, int sms, size_t static_smem,
                             Clusters clusters) {
   const double per_entry = D <= 4 ? 0.105 : (D + 8) / 75.0;
-  const double over_one = 4500, over_cluster = 5500, over_grid = 11000, over_warp = 100;
   const int num = (int)probs.size();
+  const double over_one = 4500, over_cluster = 5500, over_warp = 100;
+  // Several problems in turn take the grid 11000 to 22000 cycles a sweep
+  // beyond their entries (an iteration of 8 problems of 3400 x 3400, d = 2:
+  // 177 us, 95 in clusters of 16; 4 of 2600 x 2600: 113 and 47).
+  const double over_grid = num > 1 ? 15000 : 11000;
+  // The share of the longest problem that a batch ends with: above d = 4 large
+  // clusters gain less (64 problems of 2500 x 1000, d = 8: 360 us an iteration
+  // with 1, 230 with 0.5; 900 of 300 x 200, d = 2: 426 and 445).
+  const double tail = D > 4 ? 0.5 : 1.0;
   auto entries = [&](const RowsSize& p) { return (double)p.n * (double)p.m * per_entry; };
   // grid_t[k]: the k largest problems by the whole grid
   std::vector<double> grid_t(num + 1, 0.0);
@@ -199,8 +207,9 @@ inline RowsTeams rows_teams(const std::vector<RowsSize>& probs, int D, int sms, 
           sum += t;
           longest = std::max(longest, t);
           // problems stop at different iterations: a batch ends with its
-          // longest-running ones
-          const double est = num - k == 1 ? t : std::max(longest, sum / slots + longest);
+          // longest-running ones, unless every problem has a cluster at once
+          const bool at_once = C == kRowsMaxCluster && num <= (int)slots;
+          const double est = at_once ? longest : std::max(longest, sum / slots + tail * longest);
           if (grid_t[k] + est < best) {
             best = grid_t[k] + est;
             T.grid = k;

@@ -99,3 +99,33 @@ def test_a_device_without_room_for_the_best_cluster(tmp_path):
 def test_route_takes_the_faster_engine(tmp_path):
   rows = ",".join("{%s}" % ",".join(map(str, c)) for c in _MEASURED)
   _run(tmp_path, "static const long long kMeasured[][6] = {%s};\n%s" % (rows, _MAIN))
+
+
+_SMALL = r"""
+#include <cstdio>
+#include <vector>
+#include "fp32_route.h"
+using namespace ottb;
+int main() {
+  auto any = [](int, int, size_t) { return 64; };
+  // a few problems: each has a cluster at once, faster than the grid in turn
+  for (auto [n, m, num] : {std::tuple{2600, 2593, 4}, {2500, 2500, 5}, {3000, 2993, 6}, {3000, 2993, 8},
+                           {3400, 3393, 6}, {2200, 2193, 4}}) {
+    const RowsTeams T = rows_teams(std::vector<RowsSize>(num, {n, m, 148}), 2, 148, 2500, any);
+    if (T.grid) printf("%d of %d x %d: %d on the grid\n", num, n, m, T.grid);
+  }
+  // many above d = 4: clusters of 16 leave too much to their ends
+  for (auto [n, m] : {std::tuple{2500, 1000}, {1900, 1500}}) {
+    const RowsTeams T = rows_teams(std::vector<RowsSize>(64, {n, m, 148}), 8, 148, 2500, any);
+    if (T.grid || T.csize >= 16) printf("64 of %d x %d: grid %d, clusters of %d\n", n, m, T.grid, T.csize);
+  }
+}
+"""
+
+
+def test_teams_of_batches(tmp_path):
+  """Batches that measured slower than by the tiled engine with other teams
+  (iterations of 4 problems of 2600 x 2593, d = 2: 77 us tiled, 112 by the
+  grid in turn, 47 in clusters; 64 of 2500 x 1000, d = 8: 313 tiled, 360 in
+  clusters of 16, 229)."""
+  _run(tmp_path, "#include <tuple>\n" + _SMALL)
